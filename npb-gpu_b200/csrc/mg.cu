@@ -3,23 +3,24 @@
 // CUDA/MG/mg.cu: main's timed loop :498-508, mg3P :1078-1133).
 //
 // Grids are cubes of side m = 2^k + 2 (one ghost layer a face), x fastest,
-// one buffer per level for u and r, v on the finest level only.  Every
-// operator is one kernel that streams its grids once:
+// one buffer per level for u and r (two for the finest u), v on the finest
+// level only.  The operators:
 //   resid   r = v - A u       (:1572-1625)  27-point, a[1] = 0
 //   psinv   u = u + C r       (:1395-1440)  27-point, c[3] = 0
 //   rprj3   s = P^T r         (:1724-1790)  full weighting onto the coarse grid
 //   interp  u (+)= P z        (:836-890)    trilinear prolongation
 //   norm2u3                   (:1201-1230)  deterministic two-level reduction
-// The 27-point operators stage their input in shared memory, plane by plane
-// along z (a ring of three planes of a 32 x 8 tile with its halo, the next
-// plane loading while the current one is computed); a thread computes one x
-// of two rows from the column sums (the reference's u1/u2 line buffers) of
-// the staged rows, and takes its x neighbours' sums from the adjacent lanes
-// by shuffles.  The periodic ghost exchange (comm3,
-// :687-716, which only copies interior values) is fused: the thread that
-// writes an interior point also writes that value into each ghost cell that
-// mirrors it.  On coarse levels the reference zeroes u and then adds the
-// prolongation; here interp assigns 0 + P z in one pass.
+// A V-cycle runs them fused: k_down (resid, rprj3) and k_up (interp, resid,
+// psinv) walk a level along z and keep the intermediate grids on the SM;
+// k_coarse runs every level up to 32^3 in one launch of a cluster.  Each
+// operator is also a kernel of its own for cgb_mg_apply (k_rprj3 serves the
+// levels between as well): the 27-point ones stage their input in shared
+// memory, plane by plane along z (a ring of three planes of a 32 x 8 tile
+// with its halo, the next plane loading while the current one is computed).
+// The periodic ghost exchange (comm3, :687-716, which only copies interior
+// values) is fused: the thread that writes an interior point also writes that
+// value into each ghost cell that mirrors it.  On coarse levels the reference
+// zeroes u and then adds the prolongation; here u' = 0 + P z in one pass.
 //
 // Arithmetic: every sum in the reference's order and no fused multiply-add
 // (this file is compiled with -fmad=false), so each grid equals the serial
@@ -61,6 +62,15 @@ struct Coef {
     double a0, a2, a3;  // resid: a[1] = 0 is left out, as the reference does
     double c0, c1, c2;  // psinv: c[3] = 0 is left out
 };
+
+// Launched with programmatic stream serialization, a kernel may start while
+// its predecessor drains: it waits here before it touches what the
+// predecessor wrote, and lets its own successor start at once.
+__device__ __forceinline__ void wait_for_predecessor()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ size_t at(int m, int i3, int i2, int i1)
 {
@@ -114,6 +124,7 @@ __global__ void __launch_bounds__(kThreadsRB) k_stencil_rb(const double *__restr
                                                            double *out, int m, Coef cf)
 {
     __shared__ double ring[3][kTileRB];
+    wait_for_predecessor();
     const int n = m - 2;
     const int tx = threadIdx.x, wy = threadIdx.y, t = wy * 32 + tx;
     const int x0 = 1 + int(blockIdx.x) * 32, y0 = 1 + int(blockIdx.y) * kRowsRB;
@@ -216,6 +227,7 @@ __global__ void __launch_bounds__(kThreadsRB) k_stencil_rb(const double *__restr
 __global__ void __launch_bounds__(32 * kRows) k_rprj3(const double *__restrict__ r, int mk, double *s,
                                                       int mj)
 {
+    wait_for_predecessor();
     const int lane = threadIdx.x & 31;
     const int j1 = 1 + int(blockIdx.x) * 32 + int(threadIdx.x);
     const int j2 = 1 + int(blockIdx.y) * kRows + int(threadIdx.y);
@@ -283,11 +295,484 @@ __global__ void __launch_bounds__(32 * kRows) k_interp(const double *__restrict_
     }
 }
 
+// ---------------------------------------------------- the fused z marches
+// The V-cycle's operators on one level, fused so that a level's grids cross
+// HBM once:
+//   k_up     u' = u + P z;  r = v - A u';  out = u' + C r   (interp, resid, psinv)
+//   k_down   r = v - A u;   s = P^T r                        (resid, rprj3)
+// u' and r stay on the SM (k_down writes r when asked).  A warp owns 64
+// consecutive x (two a lane) of two consecutive y, a CTA kW such warps; it
+// walks z, and from plane to plane a thread keeps, for its four points, what
+// the next planes' column sums need (Plane27).  Rows of neighbouring warps
+// come through shared memory, neighbouring x by shuffles.  The rows and
+// columns at the tile's edge are computed by both neighbours: of 64 x 2 kW
+// points a plane, 60 x (2 kW - 4) are the CTA's own.
+//
+// Indices F run over [0, n) with F = 0 standing for index n, whose image the
+// ghost at 0 holds, so tiles start at even F and all accesses are aligned
+// pairs; reads wrap F modulo n.  An image of F <= 1 lies at F + n (comm3).
+//
+// Every point's sums are formed in the reference's order, like the single
+// operators' above, so the grids stay bit-identical.  HBM-bound by its
+// algorithmic bytes: k_up moves 3.1 grids where interp, resid and psinv apart
+// move 8.1, k_down 2.1 (3.1 writing r) where resid and rprj3 move 4.1.  At
+// 512^3: interp, resid and psinv 443 + 793 + 811 us -> k_up 1058 us (3.2
+// TB/s); resid and rprj3 793 + 307 -> k_down 824 us, writing r.  Both now wait
+// mostly on the chain of a plane's two barriers, shuffles and dependent FP64
+// adds, at 12 to 16 warps an SM.
+constexpr int kOwnX = 60;  // own columns of a warp's 64
+// Warps a CTA (one CTA an SM), by registers: k_up holds about 160 a thread.
+// 16 warps at 128 with spills: class C 56.4 ms; two CTAs of 8: 63.0; 12: 41.3.
+constexpr int kWarpsUp = 12, kWarpsDown = 16;
+
+struct Plane27 {
+    // of the plane before the centre and of the centre plane: the sums of
+    // the rows above and below, and the points themselves; [row][column]
+    double em[2][2], e0[2][2], cm[2][2], c0[2][2];
+
+    // A new plane `p` of own rows, with the rows above (`up`) and below
+    // (`dn`): the reference's column sums u1 and u2 around the centre plane,
+    // then the new plane is the centre.
+    __device__ __forceinline__ void step(const double (&p)[2][2], const double (&up)[2], const double (&dn)[2],
+                                         double (&s1)[2][2], double (&s2)[2][2])
+    {
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const double lo = i ? p[0][k] : up[k], hi = i ? dn[k] : p[1][k];
+                s1[i][k] = e0[i][k] + cm[i][k] + p[i][k];
+                s2[i][k] = em[i][k] + lo + hi;
+                em[i][k] = e0[i][k];
+                e0[i][k] = lo + hi;
+                cm[i][k] = c0[i][k];
+                c0[i][k] = p[i][k];
+            }
+    }
+};
+
+__device__ __forceinline__ int wrap(int f, int n)
+{
+    f %= n;
+    return f < 0 ? f + n : f;
+}
+
+// The values left of column 0 and right of column 1 of a lane's pair: the
+// left neighbour's column 1 and the right neighbour's column 0.
+__device__ __forceinline__ double from_left(double v1) { return __shfl_up_sync(0xffffffffu, v1, 1); }
+__device__ __forceinline__ double from_right(double v0) { return __shfl_down_sync(0xffffffffu, v0, 1); }
+
+// r = w - A u at a lane's pair of one row
+__device__ __forceinline__ void resid_pair(const double (&ctr)[2], const double (&s1)[2], const double (&s2)[2],
+                                           const double (&w)[2], const Coef &cf, double (&r)[2])
+{
+    const double s1l = from_left(s1[1]), s2l = from_left(s2[1]), s1r = from_right(s1[0]), s2r = from_right(s2[0]);
+    r[0] = w[0] - cf.a0 * ctr[0] - cf.a2 * (s2[0] + s1l + s1[1]) - cf.a3 * (s2l + s2[1]);
+    r[1] = w[1] - cf.a0 * ctr[1] - cf.a2 * (s2[1] + s1[0] + s1r) - cf.a3 * (s2[0] + s2r);
+}
+
+// u + C r at a lane's pair of one row
+__device__ __forceinline__ void psinv_pair(const double (&ctr)[2], const double (&s1)[2], const double (&s2)[2],
+                                           const double (&u)[2], const Coef &cf, double (&o)[2])
+{
+    const double s1l = from_left(s1[1]), cl = from_left(ctr[1]), s1r = from_right(s1[0]), cr = from_right(ctr[0]);
+    o[0] = u[0] + cf.c0 * ctr[0] + cf.c1 * (cl + ctr[1] + s1[0]) + cf.c2 * (s2[0] + s1l + s1[1]);
+    o[1] = u[1] + cf.c0 * ctr[1] + cf.c1 * (ctr[0] + cr + s1[1]) + cf.c2 * (s2[1] + s1[0] + s1r);
+}
+
+// A thread's place in a march: warp rows Fy, Fy + 1 and lane columns Fx,
+// Fx + 1, the wrapped offset of the first in a plane, and which are its own.
+struct March {
+    int fx, fy;
+    size_t row;  // offset of (Fy, Fx), wrapped, in a plane; the next row is m further
+    bool own;
+};
+
+template <int W>
+__device__ __forceinline__ March march_of(int m)
+{
+    const int n = m - 2, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    March q;
+    q.fx = int(blockIdx.x) * kOwnX - 2 + 2 * lane;
+    q.fy = int(blockIdx.y) * (2 * W - 4) - 2 + 2 * w;
+    q.row = size_t(wrap(q.fy, n)) * m + wrap(q.fx, n);
+    q.own = lane >= 1 && lane <= 30 && w >= 1 && w <= W - 2 && q.fx < n && q.fy < n;
+    return q;
+}
+
+// The rows v of own points of plane Fz, and their images.
+__device__ __forceinline__ void store_rows(double *g, int m, const March &q, int fz, const double (&v)[2][2])
+{
+    const int n = m - 2;
+    const size_t plane = size_t(m) * m;
+    for (int z = fz; z < m; z += n) {
+        for (int y = q.fy; y < m; y += n) {
+            double *p = g + z * plane + size_t(y) * m;
+            for (int x = q.fx; x < m; x += n) {
+                *reinterpret_cast<double2 *>(p + x) = make_double2(v[0][0], v[0][1]);
+                *reinterpret_cast<double2 *>(p + m + x) = make_double2(v[1][0], v[1][1]);
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void load_rows(const double *g, size_t plane_row, int m, double (&v)[2][2])
+{
+    const double2 a = *reinterpret_cast<const double2 *>(g + plane_row);
+    const double2 b = *reinterpret_cast<const double2 *>(g + plane_row + m);
+    v[0][0] = a.x;
+    v[0][1] = a.y;
+    v[1][0] = b.x;
+    v[1][1] = b.y;
+}
+
+// Rows through shared memory: row index 2 w + i of the CTA's 2 W rows.
+__device__ __forceinline__ void put_rows(double2 (*s)[32], const double (&v)[2][2])
+{
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    s[2 * w][lane] = make_double2(v[0][0], v[0][1]);
+    s[2 * w + 1][lane] = make_double2(v[1][0], v[1][1]);
+}
+__device__ __forceinline__ void get_row(double2 (*s)[32], int row, int rows, double (&v)[2])
+{
+    const double2 t = s[min(max(row, 0), rows - 1)][threadIdx.x & 31];
+    v[0] = t.x;
+    v[1] = t.y;
+}
+
+// kAdd: u' = u + P z (the finest level); else u' = 0 + P z.  v: the
+// right-hand side (coarse levels: the restricted residual).  u and out are
+// different arrays.  zc: own planes a CTA walks (even).
+template <int W, bool kAdd>
+__global__ void __launch_bounds__(32 * W, 1)
+    k_up(const double *z, int mj, const double *u, const double *v, double *out, int m, int zc, Coef cf)
+{
+    __shared__ double2 su[2 * W][32], sr[2 * W][32];
+    wait_for_predecessor();
+    const int n = m - 2, w = threadIdx.x >> 5;
+    const March q = march_of<W>(m);
+    const size_t plane = size_t(m) * m, zplane = size_t(mj) * mj;
+    const int z0 = int(blockIdx.z) * zc, z1 = min(n, z0 + zc);
+    const size_t zrow = size_t(wrap(q.fy, n) / 2) * mj + wrap(q.fx, n) / 2;
+    // the coarse plane i3: z[i2][i1], z[i2][i1+1], z[i2+1][i1], z[i2+1][i1+1]
+    auto coarse = [&](int i3, double (&c)[4]) {
+        const double *p = z + i3 * zplane + zrow;
+        c[0] = p[0];
+        c[1] = p[1];
+        c[2] = p[mj];
+        c[3] = p[mj + 1];
+    };
+    Plane27 U{}, R{};
+    double un[2][2] = {}, vn[2][2] = {}, za[4], zb[4] = {};
+    coarse(wrap(z0 - 2, n) / 2, za);
+    if (kAdd) load_rows(u, wrap(z0 - 2, n) * plane + q.row, m, un);
+    for (int pz = z0 - 2; pz <= z1 + 1; pz++) {
+        // u' of plane pz (interp's sums, :836-890)
+        double p[2][2];
+        {
+            const double z1a = za[2] + za[0], z1b = za[3] + za[1];
+            double add[2][2];
+            if ((pz & 1) == 0) {
+                add[0][0] = za[0];
+                add[0][1] = 0.5 * (za[1] + za[0]);
+                add[1][0] = 0.5 * z1a;
+                add[1][1] = 0.25 * (z1a + z1b);
+            } else {
+                const double z2a = zb[0] + za[0], z2b = zb[1] + za[1];
+                const double z3a = zb[2] + zb[0] + z1a, z3b = zb[3] + zb[1] + z1b;
+                add[0][0] = 0.5 * z2a;
+                add[0][1] = 0.25 * (z2a + z2b);
+                add[1][0] = 0.25 * z3a;
+                add[1][1] = 0.125 * (z3a + z3b);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int k = 0; k < 2; k++) p[i][k] = (kAdd ? un[i][k] : 0.0) + add[i][k];
+        }
+        // loads of the next plane, in flight during this one's work
+        double vc[2][2];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) vc[i][k] = vn[i][k];
+        if (pz <= z1) {
+            if (kAdd) load_rows(u, wrap(pz + 1, n) * plane + q.row, m, un);
+            load_rows(v, wrap(pz, n) * plane + q.row, m, vn);
+            if ((pz & 1) == 0) {
+                coarse(wrap(pz, n) / 2 + 1, zb);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) za[k] = zb[k];
+            }
+        }
+        double up[2], dn[2], s1[2][2], s2[2][2], uc[2][2], r[2][2], o[2][2];
+        put_rows(su, p);
+        __syncthreads();
+        get_row(su, 2 * w - 1, 2 * W, up);
+        get_row(su, 2 * w + 2, 2 * W, dn);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) uc[i][k] = U.cm[i][k];  // u' of plane pz - 2
+        U.step(p, up, dn, s1, s2);
+#pragma unroll
+        for (int i = 0; i < 2; i++) resid_pair(U.cm[i], s1[i], s2[i], vc[i], cf, r[i]);  // plane pz - 1
+        put_rows(sr, r);
+        __syncthreads();
+        get_row(sr, 2 * w - 1, 2 * W, up);
+        get_row(sr, 2 * w + 2, 2 * W, dn);
+        R.step(r, up, dn, s1, s2);
+#pragma unroll
+        for (int i = 0; i < 2; i++) psinv_pair(R.cm[i], s1[i], s2[i], uc[i], cf, o[i]);  // plane pz - 2
+        if (pz - 2 >= z0 && q.own) store_rows(out, m, q, pz - 2, o);
+    }
+}
+
+// r = v - A u, s (side mj) = its restriction, and r itself when kStore.
+template <int W, bool kStore>
+__global__ void __launch_bounds__(32 * W, 1)
+    k_down(const double *u, const double *v, double *rout, int m, double *s, int mj, int zc, Coef cf)
+{
+    __shared__ double2 su[2 * W][32], sr[2 * W][32];
+    wait_for_predecessor();
+    const int n = m - 2, nj = mj - 2, w = threadIdx.x >> 5;
+    const March q = march_of<W>(m);
+    const size_t plane = size_t(m) * m;
+    const int z0 = int(blockIdx.z) * zc, z1 = min(n, z0 + zc);
+    Plane27 U{};
+    double un[2][2], vn[2][2] = {};
+    // of the odd plane before: the rows above, at and below the coarse row;
+    // of the even plane: their sum above and below, and the centre
+    double mlo[2] = {}, mc[2] = {}, mhi[2] = {}, e0[2] = {}, ec[2] = {};
+    load_rows(u, wrap(z0 - 2, n) * plane + q.row, m, un);
+    for (int pz = z0 - 2; pz <= z1; pz++) {
+        double p[2][2], vc[2][2];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                p[i][k] = un[i][k];
+                vc[i][k] = vn[i][k];
+            }
+        if (pz < z1) {
+            load_rows(u, wrap(pz + 1, n) * plane + q.row, m, un);
+            load_rows(v, wrap(pz, n) * plane + q.row, m, vn);
+        }
+        double up[2], dn[2], s1[2][2], s2[2][2], r[2][2], lo[2];
+        put_rows(su, p);
+        __syncthreads();
+        get_row(su, 2 * w - 1, 2 * W, up);
+        get_row(su, 2 * w + 2, 2 * W, dn);
+        U.step(p, up, dn, s1, s2);
+#pragma unroll
+        for (int i = 0; i < 2; i++) resid_pair(U.cm[i], s1[i], s2[i], vc[i], cf, r[i]);
+        const int rz = pz - 1;  // r's plane
+        if (kStore && rz >= z0 && q.own) store_rows(rout, m, q, rz, r);
+        sr[2 * w + 1][threadIdx.x & 31] = make_double2(r[1][0], r[1][1]);
+        __syncthreads();
+        get_row(sr, 2 * w - 1, 2 * W, lo);
+        if ((rz & 1) == 0) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                e0[k] = lo[k] + r[1][k];
+                ec[k] = r[0][k];
+            }
+            continue;
+        }
+        // rprj3's sums (:1724-1790) around plane rz - 1
+        double x[2], y[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            x[k] = e0[k] + mc[k] + r[0][k];
+            y[k] = mlo[k] + lo[k] + mhi[k] + r[1][k];
+            mlo[k] = lo[k];
+            mc[k] = r[0][k];
+            mhi[k] = r[1][k];
+        }
+        const double xl = from_left(x[1]), yl = from_left(y[1]), cl = from_left(ec[1]);
+        if (rz - 1 >= z0 && q.own) {
+            const double val = 0.5 * ec[0] + 0.25 * (cl + ec[1] + x[0]) + 0.125 * (xl + x[1] + y[0]) +
+                               0.0625 * (yl + y[1]);
+            for (int a = (rz - 1) / 2; a < mj; a += nj)
+                for (int b = q.fy / 2; b < mj; b += nj)
+                    for (int c = q.fx / 2; c < mj; c += nj) s[at(mj, a, b, c)] = val;
+        }
+    }
+}
+
+// ------------------------------------------------------ the coarse levels
+// The V-cycle below a level whose grids are a few hundred KB, as one launch:
+// a cluster of kClusterCtas CTAs walks the levels, the operators one after
+// another with a cluster barrier between (the grids stay in L2 and the
+// barrier costs well under a microsecond, where a launch each took about 4
+// us for some 0.1 us of work): 53 us a cycle in place of 20 launches, class S
+// (32^3, 4 cycles) 0.68 -> 0.26 ms.  The levels of up to 8^3 points are CTA 0's
+// alone.  With `top` the finest level is among them and the launch runs the
+// whole benchmark's `cycles` V-cycles, each with the main loop's resid.
+constexpr int kClusterCtas = 8;
+constexpr int kClusterThreads = 512;
+constexpr int kCoarseLevel = 5;     // 32^3
+constexpr int kSoloLevel = 3;       // 8^3
+
+struct CoarseArgs {
+    double *u[kCoarseLevel + 1], *r[kCoarseLevel + 1];
+    const double *v;
+    int levels, top, cycles;
+    Coef cf;
+};
+
+// Points are dealt out as columns: thread t takes x = t % n, y = t / n % n
+// and the z run t / n^2, so that a warp reads runs of x.
+struct Column {
+    int x, y, za, zb;
+};
+__device__ __forceinline__ Column column_of(int t, int threads, int n)
+{
+    const int runs = min(n, max(1, threads / (n * n)));
+    const int c = t / (n * n), len = (n + runs - 1) / runs;
+    Column q;
+    q.x = 1 + t % n;
+    q.y = 1 + t / n % n;
+    q.za = 1 + c * len;
+    q.zb = min(n, q.za + len - 1);
+    return q;
+}
+
+// resid (kPsinv false: out = w - A g) or psinv (out = out + C g) on a column
+template <bool kPsinv>
+__device__ __forceinline__ void column_stencil(const double *g, const double *w, double *out, int m, const Column &q,
+                                               const Coef &cf)
+{
+    double em[3] = {}, e0[3] = {}, cm[3] = {}, c0[3] = {};
+    for (int z = q.za - 1; z <= q.zb + 1; z++) {
+        const double *p = g + at(m, z, q.y, q.x);
+        double lo[3], c[3], hi[3], s1[3], s2[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            lo[k] = p[k - 1 - m];
+            c[k] = p[k - 1];
+            hi[k] = p[k - 1 + m];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            s1[k] = e0[k] + cm[k] + c[k];
+            s2[k] = em[k] + lo[k] + hi[k];
+            em[k] = e0[k];
+            e0[k] = lo[k] + hi[k];
+            cm[k] = c0[k];
+            c0[k] = c[k];
+        }
+        if (z - 1 < q.za) continue;
+        const size_t o = at(m, z - 1, q.y, q.x);
+        double val;
+        if constexpr (kPsinv)
+            val = out[o] + cf.c0 * cm[1] + cf.c1 * (cm[0] + cm[2] + s1[1]) + cf.c2 * (s2[1] + s1[0] + s1[2]);
+        else
+            val = w[o] - cf.a0 * cm[1] - cf.a2 * (s2[1] + s1[0] + s1[2]) - cf.a3 * (s2[0] + s2[2]);
+        store_periodic(out, m, z - 1, q.y, q.x, val);
+    }
+}
+
+__device__ __forceinline__ void restrict_point(const double *r, int mk, double *s, int mj, int j3, int j2, int j1)
+{
+    const double *p = r + at(mk, 2 * j3, 2 * j2, 2 * j1);
+    const ptrdiff_t row = mk, pl = ptrdiff_t(mk) * mk;
+    auto cross = [&](const double *c) { return c[-row] + c[row] + c[-pl] + c[pl]; };
+    auto corner = [&](const double *c) { return c[-pl - row] + c[pl - row] + c[-pl + row] + c[pl + row]; };
+    const double val = 0.5 * p[0] + 0.25 * (p[-1] + p[1] + cross(p)) + 0.125 * (cross(p - 1) + cross(p + 1) + corner(p)) +
+                       0.0625 * (corner(p - 1) + corner(p + 1));
+    store_periodic(s, mj, j3, j2, j1, val);
+}
+
+// u (side mk) at index (f3, f2, f1), ghosts included: base + P z
+__device__ __forceinline__ double interp_point(const double *z, int mj, int f3, int f2, int f1)
+{
+    const double *p = z + at(mj, f3 >> 1, f2 >> 1, f1 >> 1);
+    const ptrdiff_t row = mj, pl = ptrdiff_t(mj) * mj;
+    auto line = [&](const double *c) {  // the reference's z1, z2, z3 or the point itself
+        if (f3 & 1) return (f2 & 1) ? c[pl + row] + c[pl] + (c[row] + c[0]) : c[pl] + c[0];
+        return (f2 & 1) ? c[row] + c[0] : c[0];
+    };
+    const double scale = ((f3 & 1) ? 0.5 : 1.0) * ((f2 & 1) ? 0.5 : 1.0);
+    if ((f1 & 1) == 0) return scale * line(p);
+    // odd x adds the two lines; where line is the point itself the reference
+    // writes z[i1 + 1] + z[i1]
+    if (((f3 | f2) & 1) == 0) return 0.5 * (p[1] + p[0]);
+    return 0.5 * scale * (line(p) + line(p + 1));
+}
+
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    __threadfence();  // plain loads after it see the other CTAs' stores
+}
+
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1) k_coarse(CoarseArgs A)
+{
+    wait_for_predecessor();
+    const bool solo_cta = blockIdx.x == 0;
+    const int gt = int(blockIdx.x) * kClusterThreads + int(threadIdx.x), all = kClusterCtas * kClusterThreads;
+    // run an operator of level k by everyone, or by CTA 0 alone below
+    auto phase = [&](int k, auto op) {
+        if (k > kSoloLevel) {
+            op(gt, all);
+            cluster_sync();
+        } else {
+            if (solo_cta) op(int(threadIdx.x), kClusterThreads);
+            __syncthreads();
+        }
+    };
+    auto restricted = [&](int k) {  // level k -> k - 1
+        phase(k, [&](int t, int threads) {
+            const int nj = 1 << (k - 1);
+            for (int e = t; e < nj * nj * nj; e += threads)
+                restrict_point(A.r[k], 2 * nj + 2, A.r[k - 1], nj + 2, 1 + e / (nj * nj), 1 + e / nj % nj, 1 + e % nj);
+        });
+    };
+    auto stencil = [&](int k, bool psinv, const double *g, const double *w, double *out) {
+        phase(k, [&](int t, int threads) {
+            const int n = 1 << k;
+            const Column q = column_of(t, threads, n);
+            if (q.za > n) return;
+            if (psinv) column_stencil<true>(g, nullptr, out, n + 2, q, A.cf);
+            else column_stencil<false>(g, w, out, n + 2, q, A.cf);
+        });
+    };
+    auto prolonged = [&](int k, bool add) {  // level k - 1 -> k
+        phase(k, [&](int t, int threads) {
+            const int mk = (1 << k) + 2, mj = (1 << (k - 1)) + 2;
+            for (int e = t; e < mk * mk * mk; e += threads) {
+                const double p = interp_point(A.u[k - 1], mj, e / (mk * mk), e / mk % mk, e % mk);
+                A.u[k][e] = (add ? A.u[k][e] : 0.0) + p;
+            }
+        });
+    };
+    const int top_level = A.levels;
+    for (int cycle = 0; cycle < A.cycles; cycle++) {
+        for (int k = top_level; k >= 2; k--) restricted(k);
+        phase(1, [&](int t, int) {  // u = 0 on the coarsest level, then psinv on it
+            if (t < 64) A.u[1][t] = 0.0;
+        });
+        stencil(1, true, A.r[1], nullptr, A.u[1]);
+        for (int k = 2; k <= top_level; k++) {
+            if (k == kSoloLevel + 1) cluster_sync();  // CTA 0's levels, to everyone
+            const bool finest = A.top && k == top_level;
+            prolonged(k, finest);
+            stencil(k, false, A.u[k], finest ? A.v : A.r[k], A.r[k]);
+            stencil(k, true, A.r[k], nullptr, A.u[k]);
+            if (finest) stencil(k, false, A.u[k], A.v, A.r[k]);
+        }
+    }
+    cluster_sync();  // no CTA leaves while another's barrier is open
+}
+
 // Sum of squares and largest magnitude over the interior: block b takes
 // rows (i2, i3) b, b + grid, ... and its threads stride x (at most four
 // values of a row each: n <= 1024); the loads of four rows are issued
 // before their values are added in the thread's fixed order.  Per-block
-// tree, then the last block (ticket) adds the blocks in order.
+// tree, then the last block (ticket) adds the blocks by the same tree.
 // out[0] = sum, out[1] = max.
 constexpr int kRowsAhead = 4, kMaxPerRow = 4;
 
@@ -296,6 +781,7 @@ __global__ void __launch_bounds__(kNormThreads) k_norm(const double *__restrict_
 {
     __shared__ double ss[kNormThreads], sm[kNormThreads];
     __shared__ bool last;
+    wait_for_predecessor();
     const int n = m - 2, rows = n * n, tid = threadIdx.x;
     double s = 0.0, mx = 0.0;
     for (int row0 = blockIdx.x; row0 < rows; row0 += kRowsAhead * gridDim.x) {
@@ -318,16 +804,20 @@ __global__ void __launch_bounds__(kNormThreads) k_norm(const double *__restrict_
                 mx = fmax(mx, fabs(xv[u][j]));
             }
     }
-    ss[tid] = s;
-    sm[tid] = mx;
-    __syncthreads();
-    for (int w = kNormThreads / 2; w > 0; w >>= 1) {
-        if (tid < w) {
-            ss[tid] = ss[tid] + ss[tid + w];
-            sm[tid] = fmax(sm[tid], sm[tid + w]);
-        }
+    // thread 0: the block's sum and largest value
+    auto block_tree = [&] {
+        ss[tid] = s;
+        sm[tid] = mx;
         __syncthreads();
-    }
+        for (int w = kNormThreads / 2; w > 0; w >>= 1) {
+            if (tid < w) {
+                ss[tid] = ss[tid] + ss[tid + w];
+                sm[tid] = fmax(sm[tid], sm[tid + w]);
+            }
+            __syncthreads();
+        }
+    };
+    block_tree();
     if (tid == 0) {
         part[2 * blockIdx.x] = ss[0];
         part[2 * blockIdx.x + 1] = sm[0];
@@ -335,15 +825,17 @@ __global__ void __launch_bounds__(kNormThreads) k_norm(const double *__restrict_
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && tid == 0) {
-        __threadfence();
-        double a = 0.0, b = 0.0;
-        for (int i = 0; i < int(gridDim.x); i++) {
-            a = a + __ldcg(part + 2 * i);
-            b = fmax(b, __ldcg(part + 2 * i + 1));
-        }
-        out[0] = a;
-        out[1] = b;
+    if (!last) return;
+    __threadfence();
+    s = mx = 0.0;
+    for (int i = tid; i < int(gridDim.x); i += kNormThreads) {
+        s = s + __ldcg(part + 2 * i);
+        mx = fmax(mx, __ldcg(part + 2 * i + 1));
+    }
+    block_tree();
+    if (tid == 0) {
+        out[0] = ss[0];
+        out[1] = sm[0];
         *ticket = 0u;
     }
 }
@@ -408,10 +900,13 @@ using namespace cgb;
 using namespace cgb::mg;
 
 struct cgb_mg {
-    int device = 0, lt = 0, smoother = 0;
+    int device = 0, lt = 0, smoother = 0, sms = 0;
     int m[kMaxLevels + 1] = {};
     double *u[kMaxLevels + 1] = {}, *r[kMaxLevels + 1] = {};
     double *v = nullptr;
+    // the finest level's other u: k_up reads one and writes the other, so the
+    // result of `graph_nit` cycles is u_now
+    double *u_other = nullptr, *u_now = nullptr;
     double *d_part = nullptr, *d_norm = nullptr;
     unsigned *d_ticket = nullptr;
     int plus[30] = {}, minus[30] = {};
@@ -455,7 +950,7 @@ void mg_release(cgb_mg *g)
         if (g->u[k]) cudaFree(g->u[k]);
         if (g->r[k]) cudaFree(g->r[k]);
     }
-    for (void *p : {(void *)g->v, (void *)g->d_part, (void *)g->d_norm, (void *)g->d_ticket})
+    for (void *p : {(void *)g->v, (void *)g->u_other, (void *)g->d_part, (void *)g->d_norm, (void *)g->d_ticket})
         if (p) cudaFree(p);
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
@@ -482,50 +977,113 @@ dim3 stencil_rb_grid(int m)
     return dim3(unsigned((n + 31) / 32), unsigned((n + kRowsRB - 1) / kRowsRB), unsigned((n + kPlanes - 1) / kPlanes));
 }
 
-void launch_resid(cgb_mg *g, int k, const double *u, const double *v, double *r)
+// A launch that may start while its predecessor drains (the kernel begins
+// with wait_for_predecessor()).
+template <typename... P, typename... A>
+void launch(cgb_mg *g, void (*k)(P...), dim3 grid, dim3 block, A... args)
 {
-    k_stencil_rb<false><<<stencil_rb_grid(g->m[k]), dim3(32, kWarpsRB), 0, g->stream>>>(u, v, r, g->m[k], g->cf);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = g->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
-void launch_psinv(cgb_mg *g, int k, const double *r, double *u)
+// The grid of a march over a level, and the own planes a CTA walks: the
+// split along z with the fewest planes on the longest SM, counting the four
+// (k_up) or two (k_down) extra planes of every walk.
+dim3 march_grid(const cgb_mg *g, int m, int warps, int extra, int *zc)
 {
-    k_stencil_rb<true><<<stencil_rb_grid(g->m[k]), dim3(32, kWarpsRB), 0, g->stream>>>(r, nullptr, u, g->m[k], g->cf);
+    const int n = m - 2, gx = (n + kOwnX - 1) / kOwnX, gy = (n + 2 * warps - 5) / (2 * warps - 4);
+    long long best = 0;
+    int best_zc = 2;
+    for (int c = 2; c <= n; c += 2) {
+        const long long chunks = (n + c - 1) / c, waves = (gx * gy * chunks + g->sms - 1) / g->sms;
+        const long long cost = waves * (c + extra);
+        if (c == 2 || cost <= best) {
+            best = cost;
+            best_zc = c;
+        }
+    }
+    *zc = best_zc;
+    return dim3(unsigned(gx), unsigned(gy), unsigned((n + best_zc - 1) / best_zc));
 }
 
-void launch_rprj3(cgb_mg *g, int k)  // level k -> k - 1
+// r[lt] (when `store`) and r[lt - 1] from the finest u and v
+void launch_down(cgb_mg *g, const double *u, bool store)
 {
-    const int mj = g->m[k - 1];
-    k_rprj3<<<stencil_grid(mj), dim3(32, kRows), 0, g->stream>>>(g->r[k], g->m[k], g->r[k - 1], mj);
+    const int lt = g->lt, m = g->m[lt];
+    int zc = 0;
+    const dim3 grid = march_grid(g, m, kWarpsDown, 2, &zc);
+    launch(g, store ? k_down<kWarpsDown, true> : k_down<kWarpsDown, false>, grid, dim3(32 * kWarpsDown), u, g->v,
+           g->r[lt], m, g->r[lt - 1], g->m[lt - 1], zc, g->cf);
 }
 
-void launch_interp(cgb_mg *g, int k, int assign)  // level k - 1 -> k
+void launch_up(cgb_mg *g, int k, const double *u, const double *v, double *out)
 {
-    const int mj = g->m[k - 1];
-    k_interp<<<interp_grid(mj), dim3(32, kRows), 0, g->stream>>>(g->u[k - 1], mj, g->u[k], g->m[k], assign);
+    const int m = g->m[k];
+    int zc = 0;
+    const dim3 grid = march_grid(g, m, kWarpsUp, 4, &zc);
+    launch(g, u ? k_up<kWarpsUp, true> : k_up<kWarpsUp, false>, grid, dim3(32 * kWarpsUp), g->u[k - 1], g->m[k - 1],
+           u, v, out, m, zc, g->cf);
+}
+
+void launch_coarse(cgb_mg *g, int levels, int top, int cycles)
+{
+    CoarseArgs A{};
+    for (int k = 1; k <= levels; k++) {
+        A.u[k] = g->u[k];
+        A.r[k] = g->r[k];
+    }
+    A.v = g->v;
+    A.levels = levels;
+    A.top = top;
+    A.cycles = cycles;
+    A.cf = g->cf;
+    launch(g, k_coarse, dim3(kClusterCtas), dim3(kClusterThreads), A);
 }
 
 void launch_norm(cgb_mg *g)
 {
-    k_norm<<<kNormBlocks, kNormThreads, 0, g->stream>>>(g->r[g->lt], g->m[g->lt], g->d_part, g->d_ticket,
-                                                        g->d_norm);
+    const int n = g->m[g->lt] - 2;
+    launch(g, k_norm, dim3(unsigned(std::min(kNormBlocks, (n * n + kRowsAhead - 1) / kRowsAhead))), dim3(kNormThreads),
+           g->r[g->lt], g->m[g->lt], g->d_part, g->d_ticket, g->d_norm);
 }
 
-// One V-cycle (mg3P, :1078-1133) then the main loop's resid.
-void enqueue_iteration(cgb_mg *g)
+// The timed region of main (:498-508): resid, norm, nit x (V-cycle (mg3P,
+// :1078-1133), resid), norm.
+void enqueue_region(cgb_mg *g, int nit)
 {
-    const int lt = g->lt;
-    for (int k = lt; k >= 2; k--) launch_rprj3(g, k);
-    cudaMemsetAsync(g->u[1], 0, sizeof(double) * cells(g->m[1]), g->stream);
-    launch_psinv(g, 1, g->r[1], g->u[1]);
-    for (int k = 2; k <= lt - 1; k++) {
-        launch_interp(g, k, 1);  // zero3 + interp
-        launch_resid(g, k, g->u[k], g->r[k], g->r[k]);
-        launch_psinv(g, k, g->r[k], g->u[k]);
+    const int lt = g->lt, m = g->m[lt];
+    g->u_now = g->u[lt];
+    if (lt <= kCoarseLevel) {
+        k_stencil_rb<false><<<stencil_rb_grid(m), dim3(32, kWarpsRB), 0, g->stream>>>(g->u[lt], g->v, g->r[lt], m,
+                                                                                      g->cf);
+        launch_norm(g);
+        if (nit > 0) launch_coarse(g, lt, 1, nit);
+        launch_norm(g);
+        return;
     }
-    launch_interp(g, lt, 0);
-    launch_resid(g, lt, g->u[lt], g->v, g->r[lt]);
-    launch_psinv(g, lt, g->r[lt], g->u[lt]);
-    launch_resid(g, lt, g->u[lt], g->v, g->r[lt]);
+    launch_down(g, g->u_now, true);
+    launch_norm(g);
+    for (int it = 0; it < nit; it++) {
+        for (int k = lt - 1; k > kCoarseLevel; k--) {
+            const int mj = g->m[k - 1];
+            launch(g, k_rprj3, stencil_grid(mj), dim3(32, kRows), g->r[k], g->m[k], g->r[k - 1], mj);
+        }
+        launch_coarse(g, kCoarseLevel, 0, 1);
+        for (int k = kCoarseLevel + 1; k < lt; k++) launch_up(g, k, nullptr, g->r[k], g->u[k]);
+        double *next = g->u_now == g->u[lt] ? g->u_other : g->u[lt];
+        launch_up(g, lt, g->u_now, g->v, next);
+        g->u_now = next;
+        launch_down(g, g->u_now, it + 1 == nit);
+    }
+    launch_norm(g);
 }
 
 // zran3 on the device: the candidates, then the host's choice of the ten
@@ -663,7 +1221,12 @@ int cgb_mg_create(int device, int lt, int smoother, cgb_mg **out)
              cudaMemset(g->u[k], 0, sizeof(double) * cells(g->m[k])) == cudaSuccess &&
              cudaMemset(g->r[k], 0, sizeof(double) * cells(g->m[k])) == cudaSuccess;
     }
-    ok = ok && cudaMalloc(&g->v, sizeof(double) * cells(g->m[lt])) == cudaSuccess;
+    ok = ok && cudaMalloc(&g->v, sizeof(double) * cells(g->m[lt])) == cudaSuccess &&
+         cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
+    if (lt > kCoarseLevel)
+        ok = ok && cudaMalloc(&g->u_other, sizeof(double) * cells(g->m[lt])) == cudaSuccess &&
+             cudaMemset(g->u_other, 0, sizeof(double) * cells(g->m[lt])) == cudaSuccess;
+    g->u_now = g->u[lt];
     if (!ok) {
         mg_release(g);
         return set_error(CGB_ERR_NOMEM, "mg: device allocation failed (2^%d grid)", lt);
@@ -692,14 +1255,9 @@ int cgb_mg_run(cgb_mg *g, int nit, double *rnm2, double *rnmu, double *device_ms
         if (g->exec) cudaGraphExecDestroy(g->exec);
         g->exec = nullptr;
         g->graph_nit = -1;
-        // the timed region of main (:498-508): resid, norm, nit x (V-cycle,
-        // resid), norm -- one graph
         cudaGraph_t graph = nullptr;
         MG_TRY(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
-        launch_resid(g, lt, g->u[lt], g->v, g->r[lt]);
-        launch_norm(g);
-        for (int it = 0; it < nit; it++) enqueue_iteration(g);
-        launch_norm(g);
+        enqueue_region(g, nit);
         const cudaError_t e1 = cudaGetLastError();
         const cudaError_t e2 = cudaStreamEndCapture(g->stream, &graph);
         if (e1 != cudaSuccess || e2 != cudaSuccess) {
@@ -739,7 +1297,7 @@ int cgb_mg_read(cgb_mg *g, int which, double *out, long long count)
     const size_t need = cells(g->m[g->lt]);
     if (count < (long long)need) return set_error(CGB_ERR_CAPACITY, "mg: %zu doubles needed", need);
     MG_TRY(cudaSetDevice(g->device));
-    const double *src = which == 0 ? g->u[g->lt] : which == 1 ? g->v : g->r[g->lt];
+    const double *src = which == 0 ? g->u_now : which == 1 ? g->v : g->r[g->lt];
     MG_TRY(cudaMemcpy(out, src, sizeof(double) * need, cudaMemcpyDeviceToHost));
     return CGB_OK;
 }

@@ -76,6 +76,22 @@ def test_benchmark_grids_bitwise(cgb, oracle, cls):
     assert got["rnmu"] == want["rnmu"]
 
 
+@pytest.mark.parametrize("lt,nit,smoother", [(2, 1, 0), (3, 2, 1), (4, 3, 0), (5, 2, 1),  # k_coarse alone
+                                             (6, 1, 0), (6, 2, 1),  # marches whose wraps meet: 64 < 2 x 60 columns
+                                             (7, 3, 1), (8, 1, 0)])  # several tiles a side, ragged at the end
+def test_fused_cycles_bitwise(cgb, oracle, lt, nit, smoother):
+    """The fused marches and the coarse-level cluster form every point's sums
+    in the oracle's order: u and r with their ghosts are bit-identical after
+    an odd and an even number of cycles (k_up alternates between two u)."""
+    want = oracle.mg_run(lt, nit, smoother, grids=True)
+    with cgb.Mg(lt, smoother) as g:
+        got = g.run(nit)
+        assert np.array_equal(g.grid("u"), want["u"])
+        assert np.array_equal(g.grid("r"), want["r"])
+    assert abs(got["rnm2"] - want["rnm2"]) <= 1e-13 * want["rnm2"]
+    assert got["rnmu"] == want["rnmu"]
+
+
 @pytest.mark.parametrize("cls", ["S", "W", "A", "B", pytest.param("C", marks=pytest.mark.slow)])
 def test_class_verifies(cgb, cls):
     c = cgb.MG_CLASSES[cls]
