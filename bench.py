@@ -686,12 +686,12 @@ def ft_section(npbcg, device, rank):
     # ft.cu:418-421
     mflops = 1.0e-6 * nt * (14.8157 + 7.19641 * np.log(nt) + (5.23518 + 7.21113 * np.log(nt)) * niter) / (ms / 1e3)
     # the initial conditions (16 B a point written), the forward transform
-    # (3 passes, 32 B each), per iteration 3 passes of 32 B (the first reads
-    # u0 and writes u1), and u0 written back once (16 B)
-    algorithmic = nt * (16 + 3 * 32 + niter * 3 * 32 + 16)
+    # (3 passes, 32 B each), per iteration 2 passes of 32 B (z reads u0 and
+    # writes u1; y and x share theirs), and u0 written back once (16 B)
+    algorithmic = nt * (16 + 3 * 32 + niter * 2 * 32 + 16)
     out = {
         "what": f"NPB FT class {FT_CLASS}: {nx}x{ny}x{nz}, {niter} iterations (one shared-memory "
-                "Stockham pass an axis, evolve fused into the z pass), FP64",
+                "Stockham pass for z with evolve and one for y and x), FP64",
         "ms": ms, "mflops": mflops,
         "max_rel_err": max(npbcg.ft_verify(FT_CLASS, r["sums"]) for r in runs),
         "verified": all(npbcg.ft_verify(FT_CLASS, r["sums"]) <= npbcg.FT_VERIFY_EPSILON for r in runs),

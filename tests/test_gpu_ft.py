@@ -41,6 +41,15 @@ def test_ft_shapes_match_oracle(cgb, oracle, dims):
     check_against_oracle(cgb, oracle, *dims)
 
 
+@pytest.mark.parametrize("dims", [(128, 128, 512, 1), (1024, 128, 64, 1), (128, 1024, 64, 1), (512, 256, 64, 2)])
+def test_ft_fused_planes_match_oracle(cgb, oracle, dims):
+    """Fields beyond 100 MB take the y and x axes in one kernel (a plane's x
+    tiles wait for its y tiles): the shortest and longest sides it is compiled
+    for, few and many tiles a plane."""
+    assert 16 * dims[0] * dims[1] * dims[2] >= 100 << 20
+    check_against_oracle(cgb, oracle, *dims)
+
+
 @pytest.mark.parametrize("cls", ["S", "W", "A", "B", "C", "D"])
 def test_ft_class_verifies(cgb, cls):
     nx, ny, nz, niter = cgb.FT_CLASSES[cls]
