@@ -88,7 +88,11 @@ def test_fused_cycles_bitwise(cgb, oracle, lt, nit, smoother):
         got = g.run(nit)
         assert np.array_equal(g.grid("u"), want["u"])
         assert np.array_equal(g.grid("r"), want["r"])
-    assert abs(got["rnm2"] - want["rnm2"]) <= 1e-13 * want["rnm2"]
+    # the oracle adds m = 8^lt squares one after another: m 2^-53 of the sum at
+    # most, half of it after the root (3.5e-13 seen of 9.3e-10 at lt = 8); the
+    # kernel's tree, at most 64 roundings deep with its rows, comes on top
+    bound = (8**lt / 2 + 64) * 2.0**-53
+    assert abs(got["rnm2"] - want["rnm2"]) <= bound * want["rnm2"]
     assert got["rnmu"] == want["rnmu"]
 
 
