@@ -105,6 +105,29 @@ __device__ __forceinline__ double spmv(Spmv &sp, const OuterArgs &A, const VT *v
     return sp.template apply<VT>(A.M, v, out, dotv, A.n, A.gb.limit_ns, A.gb.status, ok);
 }
 
+// Row j of the product just computed (to `out`), once every CTA is past a
+// barrier: by column parts the sum of the row's parts, in part order.
+template <class Spmv>
+__device__ __forceinline__ double product_at(const OuterArgs &A, const double *out, int j)
+{
+    if constexpr (Spmv::kParts) {
+        double t = 0.0;
+        for (int k = 0; k < A.M.parts; k++) t += __ldcg(A.M.part_out + k * A.M.part_stride + j);
+        return t;
+    }
+    return out[j];
+}
+
+// Makes a product's rows readable by product_at where no reduction follows it:
+// a grid barrier where rows have parts of other CTAs, else the CTA's own.
+template <class Spmv>
+__device__ __forceinline__ bool product_ready(const OuterArgs &A)
+{
+    if constexpr (Spmv::kParts) return grid_barrier(A.gb);
+    __syncthreads();
+    return true;
+}
+
 // Start of a solve (shared by the bodies): z0 = 0, r0 = x, p0 = r0 (the
 // mixed body also fills p32); leaves the partial of r.r = x.x.  (CG's first
 // iterate from z0 = 0 is already the best multiple of x, the Galerkin
@@ -140,13 +163,19 @@ __device__ __forceinline__ void end_solve(Spmv &sp, const OuterArgs &A, int row0
     if (!r_true) {
         bool ok = true;
         spmv<Spmv, double>(sp, A, A.z, A.r, nullptr, ok);
-        if (!ok) return;
-        __syncthreads();
+        if (!ok || !product_ready<Spmv>(A)) return;
     }
     double res = 0.0, xz = 0.0, zz = 0.0;
     for (int j = row0 + threadIdx.x; j < row1; j += blockDim.x) {
         const double xv = A.x[j], zv = A.z[j];
-        const double dv = r_true ? A.r[j] : xv - A.r[j];
+        double rv = A.r[j];
+        if constexpr (Spmv::kParts) {
+            if (!r_true) {
+                rv = product_at<Spmv>(A, A.r, j);
+                A.r[j] = rv;
+            }
+        }
+        const double dv = r_true ? rv : xv - rv;
         res = fma(dv, dv, res);
         xz = fma(xv, zv, xz);
         zz = fma(zv, zv, zz);
@@ -413,8 +442,11 @@ __device__ __forceinline__ void outer_step_body(const OuterArgs &A)
         // z += alpha p, r -= alpha q, rho = r.r
         acc = 0.0;
         for (int j = row0 + threadIdx.x; j < row1; j += blockDim.x) {
+            const double qv = product_at<Spmv>(A, A.q, j);
+            if constexpr (Spmv::kParts)
+                if (!A.finish) A.q[j] = qv;  // conj_grad returns q
             A.z[j] = fma(alpha, A.p[j], A.z[j]);
-            const double rv = fma(-alpha, A.q[j], A.r[j]);
+            const double rv = fma(-alpha, qv, A.r[j]);
             A.r[j] = rv;
             acc = fma(rv, rv, acc);
         }
@@ -488,11 +520,10 @@ __device__ __forceinline__ void outer_step_mixed_body(const OuterArgs &A)
             // r = x - A z with the FP64 matrix (z is complete: we are past a
             // barrier), then restart: p = r
             spmv<Spmv, double>(sp, A, A.z, A.r, nullptr, ok);
-            CGB_OK_OR_RETURN(ok);
-            __syncthreads();
+            CGB_OK_OR_RETURN(ok && product_ready<Spmv>(A));
             double acc = 0.0;
             for (int j = row0 + threadIdx.x; j < row1; j += blockDim.x) {
-                const double rv = A.x[j] - A.r[j];
+                const double rv = A.x[j] - product_at<Spmv>(A, A.r, j);
                 A.r[j] = rv;
                 A.p[j] = rv;
                 A.p32[j] = float(rv);
@@ -518,7 +549,7 @@ __device__ __forceinline__ void outer_step_mixed_body(const OuterArgs &A)
         acc = 0.0;
         for (int j = row0 + threadIdx.x; j < row1; j += blockDim.x) {
             A.z[j] = fma(alpha, A.p[j], A.z[j]);
-            const double rv = fma(-alpha, A.q[j], A.r[j]);
+            const double rv = fma(-alpha, product_at<Spmv>(A, A.q, j), A.r[j]);
             A.r[j] = rv;
             acc = fma(rv, rv, acc);
         }
@@ -704,11 +735,10 @@ __device__ __forceinline__ void outer_step_pcg_body(const OuterArgs &A)
         if (refresh) {
             // r' = b' - A' z = A z - x (FP64 matrix)
             spmv<Spmv, double>(sp, A, A.z, A.r, nullptr, ok);
-            CGB_OK_OR_RETURN(ok);
-            __syncthreads();
+            CGB_OK_OR_RETURN(ok && product_ready<Spmv>(A));
             double acc = 0.0;
             for (int j = row0 + threadIdx.x; j < row1; j += blockDim.x) {
-                const double rv = A.r[j] - A.x[j];
+                const double rv = product_at<Spmv>(A, A.r, j) - A.x[j];
                 A.r[j] = rv;
                 put_r_lowp<Spmv>(A, j, rv);
                 acc = fma(rv, rv, acc);
@@ -735,7 +765,7 @@ __device__ __forceinline__ void outer_step_pcg_body(const OuterArgs &A)
             acc = 0.0;
             for (int j = row0 + threadIdx.x; j < row1; j += blockDim.x) {
                 A.z[j] = fma(alpha, A.p[j], A.z[j]);
-                const double rv = fma(alpha, A.q[j], A.r[j]);  // r' -= alpha A'p
+                const double rv = fma(alpha, product_at<Spmv>(A, A.q, j), A.r[j]);  // r' -= alpha A'p
                 A.r[j] = rv;
                 put_r_lowp<Spmv>(A, j, rv);
                 acc = fma(rv, rv, acc);
@@ -820,6 +850,17 @@ static __global__ void __launch_bounds__(kSlicedMixedBlock, 1) outer_step_mixed_
     outer_step_mixed_body<SlicedSpmvMixedPf>(A);
 }
 
+// Column-part instances (slice_shape)
+static __global__ void __launch_bounds__(kSlicedBlock, 1) outer_step_fp64_parts(OuterArgs A)
+{
+    outer_step_body<PartSpmv64>(A);
+}
+
+static __global__ void __launch_bounds__(kSlicedMixedBlock, 1) outer_step_mixed_parts(OuterArgs A)
+{
+    outer_step_mixed_body<PartSpmvMixed>(A);
+}
+
 // Row-panel instances: the sliced plan of a matrix whose rows per CTA do
 // not fit the shared accumulators (class D: 10 K rows a CTA).
 static __global__ void __launch_bounds__(kSlicedBlock, 1) outer_step_fp64_sliced_pn(OuterArgs A)
@@ -847,6 +888,11 @@ static __global__ void __launch_bounds__(kSlicedPcgBlock, 1) outer_step_pcg_slic
     outer_step_pcg_body<SlicedSpmvPcg, kLanesF>(A);
 }
 
+static __global__ void __launch_bounds__(kSlicedPcgBlock, 1) outer_step_pcg_parts(OuterArgs A)
+{
+    outer_step_pcg_body<PartSpmvPcg, kLanesF>(A);
+}
+
 static __global__ void __launch_bounds__(kSlicedPcgBlock, 1) outer_step_pcg_sliced_pn(OuterArgs A)
 {
     outer_step_pcg_body<SlicedSpmvPcgPanels, kLanesF>(A);
@@ -858,6 +904,7 @@ static __global__ void __launch_bounds__(kSlicedPcgBlock, 1) outer_step_pcg_slic
 struct SpmvArgs {
     OuterArgs A;
     unsigned *ticket;
+    unsigned *group_ticket;  // column parts: one a group, zero between launches
     double *dot;
     int fp32;  // 1: q = A32 p32
 };
@@ -879,6 +926,22 @@ __device__ __forceinline__ void spmv_dot_body(const SpmvArgs &S)
     else acc = S.fp32 ? spmv<Spmv, float>(sp, A, A.p32, A.q, A.p, ok)
                       : spmv<Spmv, double>(sp, A, A.p, A.q, A.p, ok);
     if (!ok) return;
+    if constexpr (Spmv::kParts) {
+        if (int(blockIdx.x) < A.M.part_ctas) {  // the group's last CTA adds its rows' parts
+            __threadfence();
+            __syncthreads();
+            const int group = int(blockIdx.x) / A.M.parts;
+            if (threadIdx.x == 0) last = atomicAdd(S.group_ticket + group, 1u) == unsigned(A.M.parts - 1);
+            __syncthreads();
+            if (last) {
+                __threadfence();
+                const int j1 = A.M.group_split[group + 1];
+                for (int j = A.M.group_split[group] + threadIdx.x; j < j1; j += blockDim.x)
+                    A.q[j] = product_at<Spmv>(A, A.q, j);
+                if (threadIdx.x == 0) S.group_ticket[group] = 0u;
+            }
+        }
+    }
     const double s = block_sum(acc, scratch);
     if (threadIdx.x == 0) {
         A.part[blockIdx.x] = s;
@@ -924,6 +987,16 @@ static __global__ void __launch_bounds__(kSlicedBlock, 1) spmv_dot_sliced_pf(Spm
 static __global__ void __launch_bounds__(kSlicedBlock, 1) spmv_dot_sliced32_pf(SpmvArgs S)
 {
     spmv_dot_body<SlicedSpmvPf, 2>(S);
+}
+
+static __global__ void __launch_bounds__(kSlicedBlock, 1) spmv_dot_parts(SpmvArgs S)
+{
+    spmv_dot_body<PartSpmv64, 1>(S);
+}
+
+static __global__ void __launch_bounds__(kSlicedBlock, 1) spmv_dot_parts32(SpmvArgs S)
+{
+    spmv_dot_body<PartSpmvMixed, 2>(S);
 }
 
 static __global__ void __launch_bounds__(kSlicedBlock, 1) spmv_dot_sliced_pn(SpmvArgs S)
@@ -1021,12 +1094,13 @@ __device__ __forceinline__ int chunk_row(const int *row_split, int interleave_gr
     return interleave_grid ? c + interleave_grid * li : row_split[c] + li;
 }
 
-static __global__ void slice_sort_rows(const int *__restrict__ seg, int seg_stride, int nblk,
+constexpr int kSortBlock = 256;
+static __global__ void __launch_bounds__(kSortBlock) slice_sort_rows(const int *__restrict__ seg, int seg_stride, int nblk,
                                        const int *__restrict__ row_split, int interleave_grid,
                                        int panels, int n, const int *__restrict__ chunk_slice,
                                        unsigned short *srow, int *slice_width)
 {
-    __shared__ int hist[256];
+    __shared__ int hist[256], count[kSortBlock / 32][256];
     const int pc = blockIdx.x / nblk, b = blockIdx.x % nblk;
     const int nrows = panel_rows(row_split, interleave_grid, n, panels, pc);
     const int s0 = chunk_slice[blockIdx.x], ns = chunk_slice[blockIdx.x + 1] - s0;
@@ -1049,9 +1123,27 @@ static __global__ void slice_sort_rows(const int *__restrict__ seg, int seg_stri
     }
     __syncthreads();
     unsigned short *dst = srow + size_t(s0) * 32;
-    for (int i = threadIdx.x; i < nrows; i += blockDim.x) {
-        const int pos = atomicAdd(&hist[255 - min(SEG_LEN(i), 255)], 1);
-        dst[pos] = (unsigned short)i;
+    // rows of one length stay in order, so that the slices -- and with column
+    // parts the order in which p.q is summed -- are the same every time
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t0 = 0; t0 < nrows; t0 += kSortBlock) {
+        const int i = t0 + threadIdx.x;
+        const int key = i < nrows ? 255 - min(SEG_LEN(i), 255) : 256;
+#pragma unroll
+        for (int w = 0; w < kSortBlock / 32; w++) count[w][threadIdx.x] = 0;
+        __syncthreads();
+        const unsigned same = __match_any_sync(~0u, key);
+        const int before = __popc(same & ((1u << lane) - 1u));
+        if (key < 256 && before == 0) count[warp][key] = __popc(same);
+        __syncthreads();
+        if (key < 256) {
+            int pos = hist[key] + before;
+            for (int w = 0; w < warp; w++) pos += count[w][key];
+            dst[pos] = (unsigned short)i;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kSortBlock / 32; w++) hist[threadIdx.x] += count[w][threadIdx.x];
     }
     for (int i = nrows + threadIdx.x; i < ns * 32; i += blockDim.x) dst[i] = 0xffffu;
     __syncthreads();

@@ -275,6 +275,13 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned b
         : "memory");
 }
 
+// Asks the L2 for [src, src + bytes) (16-byte aligned, a multiple of 16);
+// nothing waits for it.
+__device__ __forceinline__ void bulk_prefetch(const void *src, unsigned bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity)
 {
     uint32_t done;

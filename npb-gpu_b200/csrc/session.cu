@@ -197,6 +197,52 @@ int validate_csr(int n, const int *rowstr, const int *colidx, const double *a)
     return st ? st : validate_entries(n, rowstr, colidx, a);
 }
 
+// How the sliced copy cuts the columns: into `parts` parts of `width` columns,
+// `groups` groups of CTAs sharing rows, a CTA a part (PartSpmv); or, parts =
+// 0, into `nblk` blocks that every CTA walks for its own rows.
+struct SliceShape {
+    int parts = 0, nblk = 0, width = kSliceWidth, groups = 0;
+    bool operator==(const SliceShape &o) const
+    {
+        return parts == o.parts && nblk == o.nblk && width == o.width && groups == o.groups;
+    }
+};
+constexpr int kMaxParts = 6;
+constexpr int kMinPartRows = 1024;     // below, only the row plan
+constexpr int kPartRowsMax = 5 * kPartCols;
+constexpr double kUnevenParts = 1.25;  // largest CTA's entries over the mean: beyond, whole rows
+constexpr unsigned kAheadEntries = 24576;
+constexpr int kBurstPairs = 6;      // PartSpmv's pairs in flight a lane
+constexpr double kSliceCost = 0.25; // of a burst: a slice's metadata and the store of its rows
+static_assert(kSlicedBlock / 32 == kPartWarps && kSlicedMixedBlock == kSlicedBlock && kSlicedPcgBlock <= kSlicedBlock);
+
+// The column parts of a matrix of order n on `sms` SMs: as few as make a part fit
+// the staging, at least 3 (a group's rows should give its warps a slice each).
+// Measured (FP64, ms for 30 or 75 steps; whole rows in brackets): n = 30000: 3
+// parts 12.3, 4 12.2, 5 12.6 (14.8); n = 50000: 3 14.4, 4 14.5, 5 15.2 (18.0); n =
+// 75000: 3 62.1, 4 62.3, 5 65.8 (75.3); n = 99991: 4 19.6, 5 20.8 (26.4); n =
+// 112000: 5 39.2 (43.6); n = 120011: 5 42.6 (45.8); n = 135007: 5 47.3 (49.7).
+// Beyond 5 parts, whole rows: n = 150000 with 6 164.4 to 172.5, as the autotuner's
+// pick falls (164.1; the mixed modes would gain, 27.6 against 29.4).  Below
+// 2 kSliceWidth rows, where the stream comes from L2, 6: n =
+// 14000 5.1, as with 8 (the row plan 6.3).
+SliceShape slice_shape(int n, int sms, bool whole_rows)
+{
+    SliceShape h;
+    if (!whole_rows && n >= kMinPartRows && n <= kPartRowsMax && sms >= kMaxParts)
+        h.parts = n < 2 * kSliceWidth ? kMaxParts : std::max(3, (n + kPartCols - 1) / kPartCols);
+    h.groups = h.parts > 0 ? sms / h.parts : 0;
+    if (h.parts == 0) {
+        h.groups = std::min(sms, n);
+        h.width = kSliceWidth;
+        h.nblk = (n + kSliceWidth - 1) / kSliceWidth;
+        return h;
+    }
+    h.width = ((n + h.parts - 1) / h.parts + 31) & ~31;
+    h.nblk = h.parts;
+    return h;
+}
+
 // Row split with balanced (stored entries + a per-row allowance for the
 // vector updates) per CTA.
 void make_split(int n, const int *rowstr, int grid, std::vector<int> &split)
@@ -267,6 +313,12 @@ struct cgb_session {
     int *d_seg = nullptr;
     int seg_stride = 0;
     int nblk = 0;
+    SliceShape shape;               // how A's sliced copy cuts the columns
+    bool uneven = false;            // this matrix loads column parts unevenly: whole rows
+    int *d_group_split = nullptr;   // first row of each group of CTAs
+    unsigned *d_group_ticket = nullptr;
+    unsigned *d_part_work = nullptr;  // PartSpmv's warps' starts, for 24 warps and for 16
+    double *d_parts = nullptr;      // kMaxParts product vectors, vstride apart
     bool sorted = false;
     bool l2_marked = false;  // a solve ran with an L2 keep fraction (lines at evict_last)
     int sliced_grid = 0;   // grid the layout was built for (0: none)
@@ -281,6 +333,10 @@ struct cgb_session {
     int prec_gen = -1;             // layout_gen sf / sft were built for
 
     Plan plan;
+    // plan is plan_main, or plan_learned while the learned mode runs: on small
+    // matrices that stays on the fastest row plan, because its factors are
+    // FP32 there and BF16 in the sliced copies
+    Plan plan_main, plan_learned;
     std::vector<int> h_rowstr_copy;
     const int *h_rowstr = nullptr;
     const int *h_colidx = nullptr;
@@ -402,6 +458,10 @@ void release(cgb_session *s)
     dev_free(s->d_trace);
     dev_free(s->d_dot);
     dev_free(s->d_seg);
+    dev_free(s->d_group_split);
+    dev_free(s->d_group_ticket);
+    dev_free(s->d_part_work);
+    dev_free(s->d_parts);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -421,7 +481,14 @@ void set_slices(cgb_session *s, const SliceSet &t, MatrixView *M)
     M->slice_width = t.width;
     M->chunk_slice = t.chunk_slice ? t.chunk_slice : s->d_chunk_slice;
     M->nblk = t.blocks ? t.blocks : s->nblk;
-    M->width = t.block_cols ? t.block_cols : kSliceWidth;
+    M->width = t.block_cols ? t.block_cols : s->shape.width;
+    M->parts = t.block_cols ? 0 : s->shape.parts;  // the factor copies: whole rows
+    M->part_ctas = M->parts * s->shape.groups;
+    M->group_split = s->d_group_split;
+    M->part_work = s->d_part_work;
+    M->part_out = s->d_parts;
+    M->part_stride = s->vstride;
+    M->ahead = s->plan.prefetch ? kAheadEntries : 0u;
     M->max_rows = s->sliced_max_rows;
     M->nacc = s->sliced_nacc;
     M->interleaved = t.interleaved;
@@ -521,14 +588,17 @@ cudaError_t launch_outer(cgb_session *s, OuterKernel k, const OuterArgs &A)
 int build_segments_table(cgb_session *s)
 {
     const int n = s->n;
-    s->nblk = (n + kSliceWidth - 1) / kSliceWidth;
+    s->shape = slice_shape(n, s->prop.multiProcessorCount, s->uneven || s->opts.panel_rows > 0);
+    s->nblk = s->shape.nblk;
     s->seg_stride = (n + 31) & ~31;
     const size_t count = size_t(s->nblk + 1) * s->seg_stride;
     if (dev_reserve(&s->d_seg, &s->cap_seg, count) != cudaSuccess)
         return set_error(CGB_ERR_NOMEM, "segment table allocation failed");
+    if (s->shape.parts > 0 && !s->d_parts && dev_alloc(&s->d_parts, kMaxParts * s->vstride) != cudaSuccess)
+        return set_error(CGB_ERR_NOMEM, "product parts allocation failed");
     CUDA_TRY(cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream));
     build_segments<<<4 * s->prop.multiProcessorCount, 256, 0, s->stream>>>(
-        s->d_rowstr, s->d_colidx, n, s->nblk, kSliceWidth, s->d_seg, s->seg_stride, s->d_flag);
+        s->d_rowstr, s->d_colidx, n, s->nblk, s->shape.width, s->d_seg, s->seg_stride, s->d_flag);
     CUDA_TRY(cudaGetLastError());
     int unsorted = 0;
     CUDA_TRY(cudaMemcpyAsync(&unsorted, s->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
@@ -562,14 +632,14 @@ int chunk_table(int grid, int panels, int nblk, RowsOf rows_of, std::vector<int>
 
 // Steps 1-3 of a sliced copy of one matrix over `grid` CTAs: row order per
 // slice, slice offsets, then values (FP64 and/or FP32) and local columns.
-// `seg` is the matrix's segment table; rows are the CTAs' ranges of d_split
-// or, with `interleave`, every grid-th row.  t->chunk_slice must be set.
+// `seg` is the matrix's segment table; rows are the ranges of row_split (a
+// CTA's, or a group's) or, with `interleave`, every grid-th row.  t->chunk_slice must be set.
 template <typename ST>
-int fill_set(cgb_session *s, int grid, bool interleave, const int *seg, const int *d_colidx,
+int fill_set(cgb_session *s, int grid, bool interleave, const int *row_split, const int *seg, const int *d_colidx,
              const ST *vals, int total, bool want64, bool want32, bool want16, SliceSet *t)
 {
     const int nblk = t->blocks ? t->blocks : s->nblk;
-    const int bcols = t->block_cols ? t->block_cols : kSliceWidth;
+    const int bcols = t->block_cols ? t->block_cols : s->shape.width;
     const int nchunks = grid * t->panels * nblk;
     const int ig = interleave ? grid : 0;
     t->interleaved = interleave ? 1 : 0;
@@ -577,7 +647,7 @@ int fill_set(cgb_session *s, int grid, bool interleave, const int *seg, const in
         dev_reserve(&t->width, &t->cap_width, size_t(total)) ||
         dev_reserve(&t->off, &t->cap_off, size_t(total) + 1))
         return set_error(CGB_ERR_NOMEM, "sliced layout: metadata allocation failed");
-    slice_sort_rows<<<nchunks, 256, 0, s->stream>>>(seg, s->seg_stride, nblk, s->d_split, ig,
+    slice_sort_rows<<<nchunks, kSortBlock, 0, s->stream>>>(seg, s->seg_stride, nblk, row_split, ig,
                                                    t->panels, s->n, t->chunk_slice, t->srow,
                                                    t->width);
     CUDA_TRY(cudaGetLastError());
@@ -594,19 +664,74 @@ int fill_set(cgb_session *s, int grid, bool interleave, const int *seg, const in
         (want16 && dev_reserve(&t->sval16, &t->cap_sval16, size_t(entries) + kPad)))
         return set_error(CGB_ERR_NOMEM, "sliced layout: %u entries do not fit", entries);
     slice_fill<ST><<<4 * s->prop.multiProcessorCount, 256, 0, s->stream>>>(
-        seg, s->seg_stride, nblk, bcols, s->d_split, ig, t->panels, s->n, t->chunk_slice, nchunks,
+        seg, s->seg_stride, nblk, bcols, row_split, ig, t->panels, s->n, t->chunk_slice, nchunks,
         d_colidx, vals, t->srow, t->width, t->off, total, t->sval, t->sval32, t->sval16, t->scol);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     return CGB_OK;
 }
 
-// The sliced copy of the matrix for a row split over `grid` CTAs (one per SM).
+// Where each of a CTA's `warps` warps starts in the CTA's slices (PartSpmv),
+// warps + 1 entries a CTA, appended to *work: equal shares of bursts of `burst`
+// step pairs, a slice counting kSliceCost of a burst besides.  The smallest
+// share (in quarters) that the warps can do is found by trying.
+void plan_part_work(const unsigned *off, const int *chunk_slice, int ctas, int warps, int burst,
+                    std::vector<unsigned> *work)
+{
+    for (int c = 0; c < ctas; c++) {
+        const int s0 = chunk_slice[c], ns = chunk_slice[c + 1] - s0;
+        double total = 0.0;
+        for (int i = 0; i < ns; i++)
+            total += kSliceCost + (int((off[s0 + i + 1] - off[s0 + i]) / 64) + burst - 1) / burst;
+        std::vector<unsigned> at(size_t(warps) + 1, part_start(ns, 0));
+        for (double share = std::max(1.25, std::floor(4.0 * total / warps) / 4.0);; share += 0.25) {
+            int i = 0, m = 0;
+            for (int w = 0; w < warps; w++) {
+                at[w] = part_start(i, m);
+                double left = share;
+                while (i < ns) {
+                    const int pairs = int((off[s0 + i + 1] - off[s0 + i]) / 64) - m;
+                    const double cost = kSliceCost + (pairs + burst - 1) / burst;
+                    if (cost <= left) {
+                        left -= cost;
+                        i++;
+                        m = 0;
+                        continue;
+                    }
+                    const int take = burst * int(left - kSliceCost);  // whole bursts of this one
+                    if (take > 0) m += take;
+                    break;
+                }
+            }
+            if (i == ns) break;
+        }
+        work->insert(work->end(), at.begin(), at.end());
+    }
+}
+
+int build_sliced(cgb_session *s, int grid);
+
+// For a matrix that column parts do not suit: its sliced copy by whole rows
+// (small matrices: none, they have the row plan).
+int build_whole_rows(cgb_session *s, int grid)
+{
+    s->uneven = true;
+    s->sliced_grid = 0;
+    if (s->n < 2 * kSliceWidth) return set_error(CGB_ERR_STATE, "sliced layout: column parts do not suit this matrix");
+    if (const int st = build_segments_table(s)) return st;
+    return build_sliced(s, grid);
+}
+
+// The sliced copy of the matrix for `grid` CTAs (one per SM).
 int build_sliced(cgb_session *s, int grid)
 {
     invalidate_sliced(s);
+    const SliceShape &h = s->shape;
+    const int groups = h.parts > 0 ? h.groups : grid;
     std::vector<int> split;
-    make_split(s->n, s->h_rowstr_copy.data(), grid, split);
+    make_split(s->n, s->h_rowstr_copy.data(), groups, split);
+    for (int c = 0; c < groups && h.parts > 0; c++)  // 16-bit rows of a group
+        if (split[c + 1] - split[c] > 0xffe0) return build_whole_rows(s, grid);
     // dynamic shared memory must fit beside the kernels' static arrays
     size_t static_smem = 0;
     for (const void *k : {(const void *)outer_step_fp64_sliced, (const void *)outer_step_mixed_sliced,
@@ -615,7 +740,10 @@ int build_sliced(cgb_session *s, int grid)
                           (const void *)outer_step_mixed_sliced_pf, (const void *)spmv_dot_sliced_pf,
                           (const void *)spmv_dot_sliced32_pf, (const void *)outer_step_fp64_sliced_pn,
                           (const void *)outer_step_mixed_sliced_pn, (const void *)outer_step_pcg_sliced_pn,
-                          (const void *)spmv_dot_sliced_pn, (const void *)spmv_dot_sliced32_pn}) {
+                          (const void *)spmv_dot_sliced_pn, (const void *)spmv_dot_sliced32_pn,
+                          (const void *)outer_step_fp64_parts, (const void *)outer_step_mixed_parts,
+                          (const void *)outer_step_pcg_parts, (const void *)spmv_dot_parts,
+                          (const void *)spmv_dot_parts32}) {
         cudaFuncAttributes fa;
         CUDA_TRY(cudaFuncGetAttributes(&fa, k));
         static_smem = std::max(static_smem, size_t(fa.sharedSizeBytes));
@@ -631,8 +759,10 @@ int build_sliced(cgb_session *s, int grid)
     // accumulators: the largest row range, or the interleaved share of the
     // preconditioner's copies; a CTA whose rows exceed them walks its rows
     // in row panels (every column block once per panel)
+    // (with column parts A needs none)
     int rows_a = 0;
-    for (int c = 0; c < grid; c++) rows_a = std::max(rows_a, split[c + 1] - split[c]);
+    if (h.parts == 0)
+        for (int c = 0; c < grid; c++) rows_a = std::max(rows_a, split[c + 1] - split[c]);
     const int rows_f = interleaved_rows(s->n, 0, grid);
     const int pa = std::max(1, (rows_a + cap - 1) / cap), pf = std::max(1, (rows_f + cap - 1) / cap);
     const int max_rows = std::max((rows_a + pa - 1) / pa, (rows_f + pf - 1) / pf);
@@ -641,11 +771,11 @@ int build_sliced(cgb_session *s, int grid)
     s->prec_panels = pf;
     s->sa.panels = pa;
     std::vector<int> chunk_slice;
-    const int total = chunk_table(grid, pa, s->nblk, [&](int c) { return split[c + 1] - split[c]; },
+    const int total = chunk_table(groups, pa, s->nblk, [&](int c) { return split[c + 1] - split[c]; },
                                   chunk_slice);
     if (dev_reserve(&s->d_chunk_slice, &s->cap_chunk, chunk_slice.size()))
         return set_error(CGB_ERR_NOMEM, "sliced layout: metadata allocation failed");
-    CUDA_TRY(cudaMemcpyAsync(s->d_split, split.data(), sizeof(int) * (grid + 1), cudaMemcpyHostToDevice,
+    CUDA_TRY(cudaMemcpyAsync(s->d_group_split, split.data(), sizeof(int) * (groups + 1), cudaMemcpyHostToDevice,
                              s->stream));
     CUDA_TRY(cudaMemcpyAsync(s->d_chunk_slice, chunk_slice.data(), sizeof(int) * chunk_slice.size(),
                              cudaMemcpyHostToDevice, s->stream));
@@ -653,7 +783,7 @@ int build_sliced(cgb_session *s, int grid)
     const int st = [&] {
         SliceSet &t = s->sa;
         t.chunk_slice = s->d_chunk_slice;
-        const int r = fill_set<double>(s, grid, false, s->d_seg, s->d_colidx, s->d_a, total, true,
+        const int r = fill_set<double>(s, groups, false, s->d_group_split, s->d_seg, s->d_colidx, s->d_a, total, true,
                                        s->opts.keep_fp32_copy != 0, false, &t);
         t.chunk_slice = nullptr;
         return r;
@@ -661,6 +791,24 @@ int build_sliced(cgb_session *s, int grid)
     if (st) return st;
     s->sliced_grid = grid;
     s->layout_gen++;
+    if (h.parts > 0) {
+        // a product takes as long as its longest CTA: where the columns are so
+        // uneven (a band, an arrow) that one CTA holds a quarter more entries
+        // than the mean, whole rows are the better split
+        std::vector<unsigned> off(size_t(total) + 1);
+        CUDA_TRY(cudaMemcpyAsync(off.data(), s->sa.off, sizeof(unsigned) * off.size(), cudaMemcpyDeviceToHost,
+                                 s->stream));
+        CUDA_TRY(cudaStreamSynchronize(s->stream));
+        unsigned most = 0;
+        const int ctas = groups * h.parts;
+        for (int c = 0; c < ctas; c++) most = std::max(most, off[chunk_slice[c + 1]] - off[chunk_slice[c]]);
+        if (double(most) * ctas > kUnevenParts * double(off[total])) return build_whole_rows(s, grid);
+        std::vector<unsigned> work;
+        plan_part_work(off.data(), chunk_slice.data(), ctas, kSlicedBlock / 32, kBurstPairs, &work);
+        plan_part_work(off.data(), chunk_slice.data(), ctas, kSlicedPcgBlock / 32, kBurstPairs, &work);
+        CUDA_TRY(cudaMemcpyAsync(s->d_part_work, work.data(), sizeof(unsigned) * work.size(), cudaMemcpyHostToDevice,
+                                 s->stream));
+    }
     return CGB_OK;
 }
 
@@ -709,7 +857,7 @@ int ensure_prec_slices(cgb_session *s)
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) st = set_error(CGB_ERR_CUDA, "factor slices: %s", cudaGetErrorString(e));
         else if (unsorted) st = set_error(CGB_ERR_STATE, "factor rows not in ascending column order");
-        else st = fill_set<float>(s, grid, true, seg, cols[m], vals[m], total, false, false, true,
+        else st = fill_set<float>(s, grid, true, s->d_group_split, seg, cols[m], vals[m], total, false, false, true,
                                   sets[m]);
     }
     dev_free(seg);
@@ -741,8 +889,8 @@ bool make_plan(cgb_session *s, int kind, int lpr, Plan *pl, int prefetch = 0, in
         if (cudaFuncSetAttribute(P.spmv, cudaFuncAttributePreferredSharedMemoryCarveout, 0)) return false;
     } else if (kind == kKindSliced) {
         // 32-bit slice offsets: keep the padded copy well below 2^32 entries
-        if (!s->sorted || s->d_seg == nullptr || s->n < 2 * kSliceWidth || s->nnz > (1LL << 30))
-            return false;
+        if (!s->sorted || s->d_seg == nullptr || s->nnz > (1LL << 30)) return false;
+        if (s->n < (s->uneven ? 2 * kSliceWidth : kMinPartRows)) return false;
         const int grid = std::min(s->prop.multiProcessorCount, s->n);
         if (s->sliced_grid != grid && build_sliced(s, grid) != CGB_OK) return false;
         // more rows a CTA than the accumulators hold: the row-panel
@@ -755,10 +903,18 @@ bool make_plan(cgb_session *s, int kind, int lpr, Plan *pl, int prefetch = 0, in
         P.pcg = pp ? outer_step_pcg_sliced_pn : outer_step_pcg_sliced;
         P.spmv = pa ? spmv_dot_sliced_pn : prefetch ? spmv_dot_sliced_pf : spmv_dot_sliced;
         P.spmv32 = pa ? spmv_dot_sliced32_pn : prefetch ? spmv_dot_sliced32_pf : spmv_dot_sliced32;
+        if (s->shape.parts > 0) {
+            P.fp64 = outer_step_fp64_parts;
+            P.mixed = outer_step_mixed_parts;
+            P.pcg = outer_step_pcg_parts;
+            P.spmv = spmv_dot_parts;
+            P.spmv32 = spmv_dot_parts32;
+        }
         P.block = kSlicedBlock;
         P.block_mixed = kSlicedMixedBlock;
         P.block_pcg = kSlicedPcgBlock;
         P.smem = sliced_smem_bytes(s->sliced_max_rows, s->sliced_nacc);
+        if (s->shape.parts > 0) P.smem = std::max(P.smem, part_smem_bytes(s->shape.width));
         for (OuterKernel k : {P.fp64, P.mixed, P.pcg})
             if (raise_smem_limit(reinterpret_cast<const void *>(k), P.smem)) return false;
         for (SpmvKernel k : {P.spmv, P.spmv32})
@@ -801,11 +957,20 @@ int apply_plan(cgb_session *s, const Plan &pl)
     return CGB_OK;
 }
 
+// Makes `pl` the current plan where it is not.
+int use_plan(cgb_session *s, const Plan &pl)
+{
+    const Plan &c = s->plan;
+    if (c.kind == pl.kind && c.lpr == pl.lpr && c.grid == pl.grid && c.prefetch == pl.prefetch) return CGB_OK;
+    return apply_plan(s, pl);
+}
+
 SpmvArgs spmv_args(cgb_session *s, int fp32)
 {
     SpmvArgs S{};
     S.A = outer_args(s);
     S.ticket = s->ticket();
+    S.group_ticket = s->d_group_ticket;
     S.dot = s->d_dot;
     S.fp32 = fp32;
     return S;
@@ -920,11 +1085,15 @@ int choose_plan(cgb_session *s)
                 }
         }
     }
-    if (want == 0 || want == kKindSliced || want == kKindSlicedPrefetch) {
-        // the sliced plan with and without the L2 prefetch of each warp's
-        // next-block slices (latency-bound short chunks gain, streaming ones lose)
-        // each instance with the matrix stream kept in L2 for the budgets
-        // below (the fraction of lines at evict_last is budget / stream)
+    const bool small = s->n < 2 * kSliceWidth;
+    if (want == 0 && small) {
+        // its stream stays in L2 by itself: neither prefetch nor budget
+        add(kKindSliced, 0, 0);
+    } else if (!small && want != kKindRow) {
+        // the sliced plan with and without the L2 prefetch (column parts: of
+        // the next product's first entries; whole rows: of each warp's
+        // next-block slices), each with the matrix stream kept in L2 for the
+        // budgets below (the fraction of lines at evict_last is budget / stream)
         for (int pf = 0; pf < 2; pf++) {
             if ((pf == 1 && want == kKindSliced) || (pf == 0 && want == kKindSlicedPrefetch)) continue;
             for (double keep : {0.0, 48e6, 64e6}) {
@@ -935,7 +1104,10 @@ int choose_plan(cgb_session *s)
         }
     }
     if (cands.empty()) return set_error(CGB_ERR_INVALID, "no kernel configuration fits these options");
-    if (cands.size() == 1) return apply_plan(s, cands[0]);
+    if (cands.size() == 1) {
+        s->plan_main = s->plan_learned = cands[0];
+        return apply_plan(s, cands[0]);
+    }
     // alternating rounds, best time per candidate: the prefetch pair differs
     // by a few per cent, about what the clock drifts over one round
     std::vector<double> best(cands.size(), 1e30);
@@ -951,9 +1123,13 @@ int choose_plan(cgb_session *s)
             best[i] = std::min(best[i], ms);
         }
     }
-    size_t bi = 0;
-    for (size_t i = 1; i < cands.size(); i++)
+    size_t bi = 0, row = cands.size();
+    for (size_t i = 0; i < cands.size(); i++) {
         if (best[i] < best[bi]) bi = i;
+        if (cands[i].kind == kKindRow && (row == cands.size() || best[i] < best[row])) row = i;
+    }
+    s->plan_main = s->plan_learned = cands[bi];
+    if (small && row < cands.size()) s->plan_learned = cands[row];
     return apply_plan(s, cands[bi]);
 }
 
@@ -997,21 +1173,24 @@ int upload_matrix(cgb_session *s, const int *rowstr, const int *colidx, const do
                            s->h_rowstr_copy.size() == size_t(s->n) + 1 &&
                            std::equal(rowstr, rowstr + s->n + 1, s->h_rowstr_copy.begin());
     s->h_rowstr_copy.assign(rowstr, rowstr + s->n + 1);
-    const int kept_kind = s->plan.kind;
+    const int kept_kind = s->plan_main.kind;
     const int kept_grid = s->sliced_grid;
+    const SliceShape kept_shape = s->shape;
     invalidate_sliced(s);
     s->sorted = false;
+    s->uneven = false;
     s->nblk = 0;
-    if (s->n >= 2 * kSliceWidth) {
+    if (s->n >= (s->opts.spmv_kernel == 0 ? kMinPartRows : 2 * kSliceWidth)) {
         int st = build_segments_table(s);
         if (st) return st;
     }
-    if (same_rows && (kept_kind == kKindRow || (s->sorted && build_sliced(s, kept_grid) == CGB_OK))) {
+    if (same_rows && (kept_kind == kKindRow || (s->sorted && build_sliced(s, kept_grid) == CGB_OK &&
+                                                s->shape == kept_shape))) {
         // the captured graph stays if every launch argument is unchanged
         // (buffers reused in place); cgb_power_iterate compares them
         return CGB_OK;
     }
-    s->plan = Plan();
+    s->plan = s->plan_main = s->plan_learned = Plan();
     return choose_plan(s);
 }
 
@@ -1343,6 +1522,10 @@ int create_shell(int n, const cgb_options *opts, cgb_session **out)
     CREATE_TRY(cudaMemsetAsync(s->d_status, 0, sizeof(int), s->stream));
     CREATE_TRY(dev_alloc(&s->d_flag, 1));
     CREATE_TRY(dev_alloc(&s->d_split, size_t(s->gpad) + 1));
+    CREATE_TRY(dev_alloc(&s->d_group_split, size_t(s->gpad) + 1));
+    CREATE_TRY(dev_alloc(&s->d_group_ticket, size_t(s->gpad)));
+    CREATE_TRY(dev_alloc(&s->d_part_work, size_t(s->gpad) * 2 * (kPartWarps + 1)));
+    CREATE_TRY(cudaMemsetAsync(s->d_group_ticket, 0, sizeof(unsigned) * s->gpad, s->stream));
     CREATE_TRY(dev_alloc(&s->d_dot, 1));
 #undef CREATE_TRY
     st = ensure_trace(s, 128);
@@ -1458,6 +1641,7 @@ int cgb_conj_grad(cgb_session *s, const int *colidx, const int *rowstr, const do
         int st = cgb_upload(s, rowstr, colidx, a);
         if (st) return st;
     }
+    if (const int st = use_plan(s, s->plan_main)) return st;
     const size_t bytes = sizeof(double) * (size_t(s->n) + 1);
     CUDA_TRY(cudaMemcpyAsync(s->x(), x, bytes, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaMemsetAsync(s->d_status, 0, sizeof(int), s->stream));
@@ -1501,7 +1685,8 @@ int cgb_power_iterate(cgb_session *s, const cgb_solve_params *params, double *ze
     int st = check_params(s, P);
     if (st) return st;
     CUDA_TRY(cudaSetDevice(s->device));
-    st = ensure_trace(s, P.niter);
+    st = use_plan(s, P.mode == CGB_MODE_MIXED_LEARNED ? s->plan_learned : s->plan_main);
+    if (!st) st = ensure_trace(s, P.niter);
     if (st) return st;
     if (P.mode == CGB_MODE_MIXED_LEARNED) {
         st = ensure_prec_slices(s);
@@ -1667,6 +1852,7 @@ int cgb_time_spmv(cgb_session *s, int reps, int fp32, double *ms_per_launch)
 {
     if (!s || reps < 1 || !ms_per_launch) return set_error(CGB_ERR_INVALID, "bad arguments");
     CUDA_TRY(cudaSetDevice(s->device));
+    if (const int st = use_plan(s, s->plan_main)) return st;
     return time_plan_spmv(s, reps, fp32 ? 1 : 0, ms_per_launch);
 }
 
@@ -1674,12 +1860,12 @@ int cgb_plan_info(cgb_session *s, int *kind, int *lanes_per_row, int *grid, int 
                   long long *smem_bytes, long long *layout_entries)
 {
     if (!s) return set_error(CGB_ERR_INVALID, "session is null");
-    if (kind) *kind = s->plan.kind == kKindSliced && s->plan.prefetch ? kKindSlicedPrefetch : s->plan.kind;
-    if (lanes_per_row) *lanes_per_row = s->plan.lpr;
-    if (grid) *grid = s->plan.grid;
-    if (block) *block = s->plan.block;
-    if (smem_bytes) *smem_bytes = (long long)s->plan.smem;
-    if (layout_entries) *layout_entries = s->plan.kind == kKindSliced ? s->sa.entries : s->nnz;
+    if (kind) *kind = s->plan_main.kind == kKindSliced && s->plan_main.prefetch ? kKindSlicedPrefetch : s->plan_main.kind;
+    if (lanes_per_row) *lanes_per_row = s->plan_main.lpr;
+    if (grid) *grid = s->plan_main.grid;
+    if (block) *block = s->plan_main.block;
+    if (smem_bytes) *smem_bytes = (long long)s->plan_main.smem;
+    if (layout_entries) *layout_entries = s->plan_main.kind == kKindSliced ? s->sa.entries : s->nnz;
     return CGB_OK;
 }
 
@@ -1699,14 +1885,14 @@ int cgb_check_status(int *word)
 int cgb_plan_l2_keep(cgb_session *s, double *bytes)
 {
     if (!s || !bytes) return set_error(CGB_ERR_INVALID, "bad arguments");
-    *bytes = s->plan.kind == kKindSliced ? s->plan.l2_keep : 0.0;
+    *bytes = s->plan_main.kind == kKindSliced ? s->plan_main.l2_keep : 0.0;
     return CGB_OK;
 }
 
 int cgb_plan_panels(cgb_session *s, int *panels, int *prec_panels)
 {
     if (!s || !panels || !prec_panels) return set_error(CGB_ERR_INVALID, "bad arguments");
-    const bool sliced = s->plan.kind == kKindSliced;
+    const bool sliced = s->plan_main.kind == kKindSliced;
     *panels = sliced ? s->sa.panels : 0;
     *prec_panels = sliced ? s->prec_panels : 0;
     return CGB_OK;
@@ -1715,7 +1901,7 @@ int cgb_plan_panels(cgb_session *s, int *panels, int *prec_panels)
 int cgb_set_l2_keep(cgb_session *s, double bytes)
 {
     if (!s || !(bytes >= 0.0) || bytes > 1e12) return set_error(CGB_ERR_INVALID, "bytes must be in [0, 1e12]");
-    s->plan.l2_keep = bytes;
+    s->plan.l2_keep = s->plan_main.l2_keep = s->plan_learned.l2_keep = bytes;
     drop_graph(s);
     return CGB_OK;
 }
@@ -1726,7 +1912,8 @@ int cgb_time_outer_steps(cgb_session *s, int niter, double shift, double *kernel
     if (!s || niter < 1 || !kernel_ms || !graph_gap_ms)
         return set_error(CGB_ERR_INVALID, "bad arguments");
     CUDA_TRY(cudaSetDevice(s->device));
-    int st = ensure_trace(s, niter);
+    int st = use_plan(s, s->plan_main);
+    if (!st) st = ensure_trace(s, niter);
     if (st) return st;
     std::vector<cudaEvent_t> ev(niter + 1);
     for (auto &e : ev) CUDA_TRY(cudaEventCreate(&e));
@@ -1763,6 +1950,7 @@ int cgb_time_barrier(cgb_session *s, int iters, double *us_per_barrier)
     if (!s || iters < 1 || iters > 10000000 || !us_per_barrier)
         return set_error(CGB_ERR_INVALID, "bad arguments");
     CUDA_TRY(cudaSetDevice(s->device));
+    if (const int st = use_plan(s, s->plan_main)) return st;
     GridBarrier gb;
     gb.arrivals = s->arrivals();
     gb.status = s->d_status;

@@ -182,6 +182,19 @@ struct MatrixView {
                                               // consecutive pieces (row panels), each
                                               // over every column block: 1 unless the
                                               // rows exceed the accumulators
+    // column parts (PartSpmv): the first part_ctas CTAs form groups of `parts`;
+    // CTA c computes the rows of group c / parts (group_split) over the `width`
+    // columns of part c % parts, into the part's own vector (part_out,
+    // part_stride apart); a row's parts are added where it is used.  parts = 0:
+    // whole rows.
+    int parts, part_ctas;
+    const int *__restrict__ group_split;
+    const unsigned *__restrict__ part_work;  // where each warp starts (plan_part_work)
+    double *part_out;
+    size_t part_stride;
+    // entries of a CTA's stream asked of the L2 at the end of a product, for
+    // the next one (PartSpmv; a multiple of 64, 0: none)
+    unsigned ahead;
     // bounds of the checked build: CSR entries and sliced entries (each with
     // the padding after them), columns of the gathered vector
     long long csr_entries, slice_entries;
@@ -289,6 +302,7 @@ __device__ __forceinline__ double spmv_rows(const MatrixView &M, const VT *v, do
 template <int LPR>
 struct RowSpmv {
     static constexpr bool kSliced = false;
+    static constexpr bool kParts = false;
     int row0, row1;
     __device__ void setup(const MatrixView &, int r0, int r1)
     {
@@ -356,6 +370,7 @@ template <int kU64, int kU32, bool kOutline = false, bool kL2Prefetch = true, bo
           int kU16 = 2 * kU32>
 struct SlicedSpmvT {
     static constexpr bool kSliced = true;
+    static constexpr bool kParts = false;
     // Dynamic shared memory: the control words first (fixed offsets), then
     // the staging, then the accumulators; every address is a constant offset
     // from the array, so the policy keeps only three registers of state.
@@ -605,6 +620,188 @@ struct SlicedSpmvT {
     }
 };
 
+// The product by column parts: a CTA stages one block of the vector, its
+// part's (up to kPartCols columns, 212 KB: the accumulators' space too, which
+// only Base uses, in products of its own), and its rows' segments in those
+// columns are one chunk of slices.
+//
+// A CTA that computes whole rows stages all of the vector for every product
+// (148 x 600 KB at n = 75000, beside a matrix stream of 150 MB), in blocks
+// that cut its rows' entries into short slices, with an accumulator pass over
+// the rows at the end.  With `parts` CTAs sharing their rows, each stages its
+// part once, its slices are longer, nothing is refilled, and a lane's sum is
+// the row's part: stored from the register, and multiplied by dotv's entry,
+// which was fetched with the slice.  The parts of a row (8 bytes each) are
+// added where the product is used.
+//
+// The slices of a CTA lie one after another, widest first, and a warp takes a
+// stretch of them (part_work): every warp about as many bursts of kU step pairs
+// a lane, which is what a walk takes time by (2.5 to 2.7 us each).  A stretch may
+// begin or end inside a slice: its warps leave their sums in shared memory, and
+// the one that began it adds them, in order, after the CTA's barrier.  With whole slices dealt to the warps the longest had 15.8
+// bursts where the mean was 11.5 (n = 75000, 4 parts: 69.8 ms a solve, now 62.3).
+//
+// (Loading the pairs after while the present ones are used, in two register
+// sets, is slower: 86 to 94 ms a solve at n = 75000 against 66.)  Base: the walk
+// for the preconditioner's factor copies (whole rows).
+constexpr int kPartCols = 27136;
+constexpr int kPartWarps = 24;  // at most
+// Dynamic shared memory of a part's staging and the sums of continued slices
+__host__ __device__ inline size_t part_smem_bytes(int cols)
+{
+    return 128 + size_t(cols) * sizeof(double) + 2 * kPartWarps * 32 * sizeof(double);
+}
+// An entry of part_work: a slice (of the CTA's) and a step pair in it
+__host__ __device__ inline unsigned part_start(int slice, int pair) { return unsigned(slice) << 16 | unsigned(pair); }
+template <int kU64, int kU32, class Base>
+struct PartSpmv : Base {
+    static constexpr bool kParts = true;
+
+    template <typename VT, typename ST = VT>
+    __device__ __forceinline__ double apply(const MatrixView &M, const VT *v, double *out, const double *dotv, int n,
+                                            long long limit_ns, int *status, bool &ok)
+    {
+        if constexpr (sizeof(ST) == 2) return Base::template apply<VT, ST>(M, v, out, dotv, n, limit_ns, status, ok);
+        else return walk<VT>(M, v, dotv, n, limit_ns, status, ok);
+    }
+
+    template <typename VT>
+    __device__ __forceinline__ double walk(const MatrixView &M, const VT *v, const double *dotv, int n,
+                                           long long limit_ns, int *status, bool &ok)
+    {
+        using P2 = typename Pair<VT>::T;
+        constexpr int kU = sizeof(VT) == 8 ? kU64 : kU32;
+        ok = true;
+        if (int(blockIdx.x) >= M.part_ctas) return 0.0;
+        const VT *__restrict__ vals = slice_values<VT>(M);
+        const uint64_t pol = l2_stream_policy(sizeof(VT) == 8 ? M.keep64 : M.keep32);
+        const int part = int(blockIdx.x) % M.parts, group = int(blockIdx.x) / M.parts;
+        // (a part past the last column has no entries: it stages the first)
+        const int row0 = M.group_split[group], col0 = part * M.width < n ? part * M.width : 0;
+        double *const out = M.part_out + part * M.part_stride + row0;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        const int s0 = __ldg(M.chunk_slice + blockIdx.x), s1 = __ldg(M.chunk_slice + blockIdx.x + 1);
+        VT *const pv = reinterpret_cast<VT *>(Base::buf());
+        uint64_t *const bar = Base::bars();
+        if (threadIdx.x == 0) {
+            fence_proxy_async();  // v was written by generic stores before the grid barrier
+            const unsigned cols = unsigned(min(M.width, n - col0));
+            bulk_load(pv, v + col0, (cols * unsigned(sizeof(VT)) + 15u) & ~15u, bar);
+        }
+
+        // this warp's stretch: from pair m0 of its first slice to pair tail of
+        // slice last (none of it if 0)
+        const unsigned *work = M.part_work + (nw == kPartWarps ? 0 : M.part_ctas * (kPartWarps + 1)) +
+                               int(blockIdx.x) * (nw + 1);
+        const unsigned from = __ldg(work + warp), to = __ldg(work + warp + 1);
+        const int last = s0 + int(to >> 16), tail = int(to & 0xffffu);
+        double *const carry = reinterpret_cast<double *>(Base::buf() + size_t(M.width) * sizeof(double));
+        struct Slice {
+            unsigned off;  // this lane's first entry
+            int wp;        // step pairs to walk to; -1 past the end
+            unsigned short row;
+            double dot;
+        };
+        auto slice = [&](int s) {
+            Slice t{0u, -1, 0xffffu, 0.0};
+            if (s < last || (s == last && tail > 0)) {
+                t.off = __ldg(M.slice_off + s) + 2u * lane;
+                t.wp = s < last ? __ldg(M.slice_width + s) >> 1 : tail;
+                t.row = __ldg(M.srow + size_t(s) * 32 + lane);
+                if (dotv && t.row != 0xffffu) t.dot = __ldcg(dotv + row0 + t.row);
+            }
+            return t;
+        };
+        double dacc = 0.0;
+        int s = s0 + int(from >> 16), m0 = int(from & 0xffffu);
+        Slice cur = slice(s);
+        bool failed = false, staged = false;
+        for (; cur.wp >= 0 && !failed; s++) {
+            const Slice nxt = slice(s + 1);  // its metadata loads during this slice
+            VT sum = VT(0);
+            for (int m = m0; m < cur.wp; m += kU) {
+                P2 av[kU];
+                ushort2 cv[kU];
+#pragma unroll
+                for (int u = 0; u < kU; u++) {
+                    if (m + u < cur.wp) {
+                        const unsigned e = cur.off + 64u * unsigned(m + u);
+                        if (CGB_IN_RANGE(e + 1, M.slice_entries, kCheckStream)) {
+                            av[u] = ld_stream(reinterpret_cast<const P2 *>(vals + e), pol);
+                            cv[u] = ld_stream(reinterpret_cast<const ushort2 *>(M.scol + e), pol);
+                        } else {
+                            av[u].x = av[u].y = VT(0);
+                            cv[u] = make_ushort2(0, 0);
+                        }
+                    }
+                }
+                if (!staged) {  // the first pairs are on their way: now the vector
+                    staged = true;
+                    if (!mbar_wait(bar, this->parity & 1u, limit_ns, Base::abort_flag())) {
+                        failed = true;
+                        *Base::abort_flag() = 1;
+                        break;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kU; u++) {
+                    if (m + u < cur.wp) {
+                        if (CGB_IN_RANGE(cv[u].x, M.width, kCheckGather)) sum = fma_vt(av[u].x, pv[cv[u].x], sum);
+                        if (CGB_IN_RANGE(cv[u].y, M.width, kCheckGather)) sum = fma_vt(av[u].y, pv[cv[u].y], sum);
+                    }
+                }
+            }
+            const bool valid = cur.row != 0xffffu && CGB_IN_RANGE(row0 + cur.row, M.ncols, kCheckRow);
+            if (valid) dacc = fma(cur.dot, double(sum), dacc);
+            if (m0 > 0) carry[warp * 32 + lane] = double(sum);
+            else if (s == last) carry[(kPartWarps + warp) * 32 + lane] = double(sum);
+            else if (valid) out[cur.row] = double(sum);
+            m0 = 0;
+            cur = nxt;
+        }
+        // (a warp without entries has not waited yet: the phase must be over
+        // before the next product arms the barrier again)
+        if (!failed && !staged && !mbar_wait(bar, this->parity & 1u, limit_ns, Base::abort_flag())) {
+            failed = true;
+            *Base::abort_flag() = 1;
+        }
+        this->parity ^= 1u;
+        if (threadIdx.x == 0 && M.ahead > 0) {
+            // HBM would idle through the reductions and vector updates ahead
+            const unsigned o = __ldg(M.slice_off + s0), count = min(M.ahead, __ldg(M.slice_off + s1) - o);
+            for (unsigned k = 0; k < count; k += 4096u) {
+                const unsigned part_count = min(4096u, count - k);
+                bulk_prefetch(vals + o + k, part_count * unsigned(sizeof(VT)));
+                bulk_prefetch(M.scol + o + k, part_count * 2u);
+            }
+        }
+        // the slot's reads are over before the next product refills it
+        if (__syncthreads_or(failed)) {
+            ok = false;
+            if (threadIdx.x == 0) {
+                raise_status(status, kDevTimeout);
+                // let the issued copy land before the CTA leaves
+                (void)mbar_wait(bar, (this->parity & 1u) ^ 1u, limit_ns, nullptr);
+            }
+            __syncthreads();
+            return 0.0;
+        }
+        const unsigned begun = __ldg(work + warp), ended = __ldg(work + warp + 1);
+        if ((ended & 0xffffu) != 0u && ((begun ^ ended) >> 16 != 0u || (begun & 0xffffu) == 0u)) {
+            // the slice that this warp began and others continue
+            const unsigned short row = __ldg(M.srow + size_t(s0 + int(ended >> 16)) * 32 + lane);
+            double t = carry[(kPartWarps + warp) * 32 + lane];
+            for (int k = warp + 1; k < nw; k++) {
+                const unsigned w = __ldg(work + k);
+                if ((w ^ ended) >> 16 != 0u || (w & 0xffffu) == 0u) break;
+                t += carry[k * 32 + lane];
+            }
+            if (row != 0xffffu && CGB_IN_RANGE(row0 + row, M.ncols, kCheckRow)) out[row] = t;
+        }
+        return dacc;
+    }
+};
+
 // Per kernel (pair counts and block shapes measured on B200): the FP64
 // outer step and the standalone SpMVs (768 threads, 80 registers), the
 // mixed outer step (768), the preconditioned one (512, 128 registers).
@@ -617,5 +814,10 @@ using SlicedSpmvPcg = SlicedSpmvT<4, 10, false, false, false, 8>;
 using SlicedSpmvPanels = SlicedSpmvT<6, 6, false, false, true>;
 using SlicedSpmvMixedPanels = SlicedSpmvT<4, 6, false, false, true>;
 using SlicedSpmvPcgPanels = SlicedSpmvT<4, 6, false, false, true>;
+
+// column-part instances
+using PartSpmv64 = PartSpmv<6, 6, SlicedSpmv>;
+using PartSpmvMixed = PartSpmv<4, 6, SlicedSpmv>;
+using PartSpmvPcg = PartSpmv<4, 10, SlicedSpmvPcg>;
 
 }  // namespace cgb

@@ -357,6 +357,94 @@ def test_row_panels_change_no_result(cgb):
         assert np.all(outs[1][k]["rnorm"] <= 1e-10 * np.sqrt(n)), k  # 1e-10 ||x||, x = 1 first
 
 
+def banded(n, half, shift):
+    """A negative definite band: its rows meet few columns, so column parts
+    would leave most CTAs of a group idle."""
+    offs = np.arange(-half, half + 1)
+    cols = np.arange(n)[:, None] + offs
+    ok = (cols >= 0) & (cols < n)
+    vals = np.where(offs == 0, -float(shift), 0.25 * np.cos(cols * 0.37 + offs))
+    vals = 0.5 * (vals + np.where(offs == 0, -float(shift), 0.25 * np.cos((cols - offs) * 0.37 - offs)))
+    rs = np.zeros(n + 1, np.int32)
+    rs[1:] = np.cumsum(ok.sum(1))
+    return rs, cols[ok].astype(np.int32), vals[ok]
+
+
+@pytest.mark.parametrize("n", [24576, 30011, 75037, 81408, 81409, 135680, 135681])
+def test_column_parts_agree_with_rows(cgb, n):
+    """The sliced plan by column parts (groups of CTAs that share rows, a part
+    of the columns each) at its smallest order, odd ones, on both sides of one
+    part more, its largest and the first by whole rows: every mode's zeta agrees with the row plan's, to 1e-12
+    in FP64 (other summation orders) and to the parity bar in the tolerance
+    modes; conj_grad returns the same q = A p, p and z."""
+    rs, ci, a = cgb.makea(n, 5, 0.1, 12.0 + n / 2000.0)
+    factor = cgb.jacobi_factor(rs, ci, a)
+    x = 1.0 + 0.5 * np.sin(np.arange(n) * 0.003)
+    outs, vecs = [], []
+    for kind in (1, 2, 3):
+        with cgb.Session(rs, ci, a, spmv_kernel=kind) as s:
+            vecs.append(s.conj_grad(x))
+            shift = 12.0 + n / 2000.0
+            r = [s.power_iterate(4, shift)["zeta"],
+                 s.power_iterate(4, shift, mode=cgb.MODE_FP64_TOL, tol=1e-12, cgitmax=100)["zeta"],
+                 s.power_iterate(4, shift, mode=cgb.MODE_MIXED, tol=1e-12, cgitmax=100)["zeta"]]
+            s.set_preconditioner(*factor)
+            r.append(s.power_iterate(4, shift, mode=cgb.MODE_MIXED_LEARNED, tol=1e-12, cgitmax=100)["zeta"])
+            assert 0 < s.time_spmv(3) < 50 and 0 < s.time_spmv(3, True) < 50
+            outs.append(r)
+    for o in outs[1:]:
+        for k, bound in enumerate((1e-12, 1e-10, 1e-10, 1e-10)):
+            assert np.max(np.abs(o[k] - outs[0][k]) / np.abs(outs[0][k])) <= bound, (n, k)
+    for v in vecs[1:]:
+        assert np.linalg.norm(v[0] - vecs[0][0]) <= 1e-12 * np.linalg.norm(vecs[0][0])
+        for k in (1, 2):  # p and q: rounding noise by now, of the start's 1e-10 at most
+            assert np.linalg.norm(v[k][:n] - vecs[0][k][:n]) <= 1e-10 * np.linalg.norm(x)
+    # the prefetch of the next product's entries changes no bit
+    assert all(np.array_equal(p, q) for p, q in zip(outs[1][:3], outs[2][:3]))
+
+
+@pytest.mark.parametrize("n", [1023, 1024, 1400, 9001, 24575])
+def test_small_systems_every_mode(cgb, oracle, n):
+    """Below the sliced plan's order the autotuner also has the column parts (6
+    of them): whatever it picks, zeta and z agree with the oracle's, and a
+    learned solve between two FP64 ones (which may run on another plan) changes
+    neither."""
+    shift = 12.0 + n / 2000.0
+    rs, ci, a = cgb.makea(n, 6, 0.1, shift)
+    zo, *_ = oracle.conj_grad(rs, ci, a, np.ones(n))
+    with cgb.Session(rs, ci, a) as s:
+        z = s.conj_grad(np.ones(n))[0]
+        first = s.power_iterate(3, shift)["zeta"]
+        mixed = s.power_iterate(3, shift, mode=cgb.MODE_MIXED, tol=1e-12, cgitmax=100)["zeta"]
+        s.set_preconditioner(*cgb.jacobi_factor(rs, ci, a))
+        learned = s.power_iterate(3, shift, mode=cgb.MODE_MIXED_LEARNED, tol=1e-12, cgitmax=100)["zeta"]
+        again = s.power_iterate(3, shift)["zeta"]
+        assert s.plan()["kind"] in ("row", "sliced")
+    assert np.linalg.norm(z[:n] - zo[:n]) <= 1e-12 * np.linalg.norm(zo[:n])
+    assert np.array_equal(first, again)
+    for other in (mixed, learned):
+        assert np.max(np.abs(other - first) / np.abs(first)) <= 1e-10
+
+
+def test_uneven_columns_take_whole_rows(cgb):
+    """A band at an order the column parts would take: whole rows (as before
+    them) where the sliced plan is asked for, and the row plan's result."""
+    n = 30000
+    rs, ci, a = banded(n, 6, 8.0)
+    out = {}
+    for kind in (1, 2):
+        with cgb.Session(rs, ci, a, spmv_kernel=kind) as s:
+            out[kind] = s.power_iterate(3, 8.0)["zeta"]
+            if kind == 2:
+                assert s.plan()["kind"] == "sliced" and s.plan()["grid"] >= 148
+                s.upload(rs, ci, a * 2.0)  # the same rows again: the copy is rebuilt, still by whole rows
+                doubled = s.power_iterate(3, 8.0)["zeta"]
+    assert np.max(np.abs(out[1] - out[2]) / np.abs(out[1])) <= 1e-12
+    with cgb.Session(rs, ci, a * 2.0, spmv_kernel=1) as s:
+        ref = s.power_iterate(3, 8.0)["zeta"]
+    assert np.max(np.abs(doubled - ref) / np.abs(ref)) <= 1e-12
+
+
 def test_class_d_sliced_row_panels(cgb):
     """Class D (n = 1.5 M, 694 M entries; 10 K rows a CTA) on the sliced
     plan walks row panels; its first outer steps agree with the row plan's
