@@ -30,6 +30,7 @@ constexpr int kF = 4;      // input features
 constexpr int kL = 3;      // message-passing layers
 constexpr int kK = 32;     // probe vectors per training step
 constexpr int kRedBlocks = 256;  // CTAs of the row reductions
+constexpr int kHeadBlocks = 592;  // CTAs of the head backward (a gather an entry: four CTAs an SM)
 
 // Offsets of the flat parameter vector (see oracle/gnn_oracle.py).
 constexpr int kOffWin = 0;
@@ -53,10 +54,9 @@ __device__ __forceinline__ float softplus_f(float u) { return u > 20.f ? u : log
 __device__ __forceinline__ float sigmoid_f(float u) { return 1.f / (1.f + expf(-u)); }
 
 // ----------------------------------------------------------------- forward
-// out[i,:] = act(in[i,:in_dim] W + b (+ add[i,:])), W in_dim x 32 row-major.
+// out[i,:] = act(in[i,:in_dim] W + b), W in_dim x 32 row-major.
 __global__ void k_dense(const float *__restrict__ in, int in_dim, const float *__restrict__ W,
-                        const float *__restrict__ b, const float *__restrict__ add, float *out,
-                        int n, int relu)
+                        const float *__restrict__ b, float *out, int n, int relu)
 {
     __shared__ float sW[kH * kH];
     for (int t = threadIdx.x; t < in_dim * kH; t += blockDim.x) sW[t] = W[t];
@@ -68,65 +68,135 @@ __global__ void k_dense(const float *__restrict__ in, int in_dim, const float *_
         const float xi = lane < in_dim ? in[size_t(i) * in_dim + lane] : 0.f;
         float acc = bc;
         for (int k = 0; k < in_dim; k++) acc = fmaf(__shfl_sync(0xffffffffu, xi, k), sW[k * kH + lane], acc);
-        if (add) acc += add[size_t(i) * kH + lane];
         out[size_t(i) * kH + lane] = relu ? fmaxf(acc, 0.f) : acc;
     }
 }
 
-// out[i,:] = in1[i,:] W1^T + in2[i,:] W2^T (both 32 x 32; in2/W2 optional).
-__global__ void k_dense_t2(const float *__restrict__ in1, const float *__restrict__ W1,
-                           const float *__restrict__ in2, const float *__restrict__ W2, float *out,
-                           int n)
+constexpr int kAhead = 8;  // gathers a warp has in flight
+
+// Row i of a sparse product on a block of 32 columns, lane c its column c:
+// sum_k w_k in[col_k, c] from acc on, in stored order, w_k = val[k] or
+// val[map[k]] (map may be null).  The gathers of kAhead entries are in flight
+// at once: one at a time, a row is a chain of L2 round trips.
+__device__ __forceinline__ float spmm_row(int k0, int k1, const int *__restrict__ col,
+                                          const float *__restrict__ val, const int *__restrict__ map,
+                                          const float *__restrict__ in, int lane, float acc)
+{
+    for (int k = k0; k < k1; k += kAhead) {
+        float w[kAhead], x[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            if (k + u < k1) {
+                w[u] = map ? val[map[k + u]] : val[k + u];
+                x[u] = in[size_t(col[k + u]) * kH + lane];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+            if (k + u < k1) acc = fmaf(w[u], x[u], acc);
+    }
+    return acc;
+}
+
+// out[i,:] = cscale * (diag[i] in[i,:] + sum_k w_k in[col_k,:] - sub[i,:]);
+// sub and the column factors cscale may be null.
+__global__ void k_spmm(const int *__restrict__ ptr, const int *__restrict__ col,
+                       const float *__restrict__ val, const int *__restrict__ map,
+                       const float *__restrict__ diag, const float *__restrict__ in,
+                       const float *__restrict__ sub, const float *__restrict__ cscale, float *out, int n)
+{
+    const int lane = threadIdx.x & 31;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
+         i += (gridDim.x * blockDim.x) >> 5) {
+        const size_t at = size_t(i) * kH + lane;
+        float acc = spmm_row(ptr[i], ptr[i + 1], col, val, map, in, lane, diag[i] * in[at]);
+        if (sub) acc -= sub[at];
+        if (cscale) acc *= cscale[lane];
+        out[at] = acc;
+    }
+}
+
+// The row of a 32-column block (lane c its column c) times W (32 x 32 in
+// shared memory, sW[k * kH + c]), from acc on.
+__device__ __forceinline__ float row_times(float x, const float *sW, int lane, float acc)
+{
+#pragma unroll 8
+    for (int k = 0; k < kH; k++) acc = fmaf(__shfl_sync(0xffffffffu, x, k), sW[k * kH + lane], acc);
+    return acc;
+}
+
+// One message-passing layer: H' = relu(H Ws + b + Aoff T), and T' = H' Wm' of
+// the next layer (Wm_next may be null): a row's whole way through the layer
+// in its warp's registers.
+__global__ void k_layer(const float *__restrict__ H, const float *__restrict__ T, const float *__restrict__ Ws,
+                        const float *__restrict__ b, const int *__restrict__ ptr, const int *__restrict__ col,
+                        const float *__restrict__ val, const float *__restrict__ Wm_next, float *H_out, float *T_out,
+                        int n)
 {
     __shared__ float s1[kH * kH], s2[kH * kH];
     for (int t = threadIdx.x; t < kH * kH; t += blockDim.x) {
-        s1[t] = W1[t];
-        s2[t] = W2 ? W2[t] : 0.f;
+        s1[t] = Ws[t];
+        s2[t] = Wm_next ? Wm_next[t] : 0.f;
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
          i += (gridDim.x * blockDim.x) >> 5) {
-        const float a1 = in1[size_t(i) * kH + lane];
-        const float a2 = in2 ? in2[size_t(i) * kH + lane] : 0.f;
-        float acc = 0.f;
-        for (int k = 0; k < kH; k++) {
-            acc = fmaf(__shfl_sync(0xffffffffu, a1, k), s1[lane * kH + k], acc);
-            if (in2) acc = fmaf(__shfl_sync(0xffffffffu, a2, k), s2[lane * kH + k], acc);
-        }
-        out[size_t(i) * kH + lane] = acc;
+        const size_t at = size_t(i) * kH + lane;
+        const float u = spmm_row(ptr[i], ptr[i + 1], col, val, nullptr, T, lane, 0.f);
+        const float h = fmaxf(row_times(H[at], s1, lane, b[lane]) + u, 0.f);
+        H_out[at] = h;
+        if (Wm_next) T_out[at] = row_times(h, s2, lane, 0.f);
     }
 }
 
-// out[i,:] = dscale*in[i,:] + sum_k w_k in[col_k,:], w_k = val[k] or
-// val[map[k]] (map may be null); diag may be null (then the row's own term
-// is diag_const * in[i,:]).
-__global__ void k_spmm(const int *__restrict__ ptr, const int *__restrict__ col,
-                       const float *__restrict__ val, const int *__restrict__ map,
-                       const float *__restrict__ diag, float diag_const,
-                       const float *__restrict__ in, float *out, int n)
+// The same layer backward, from dz (masked): dT = Aoff dz, and the next
+// dz' = (dz Ws^T + dT Wm^T) where h > 0.  The weights are staged transposed:
+// lane c reads their row c, and rows of 32 floats would all start on bank 0.
+__global__ void k_layer_bwd(const float *__restrict__ dz, const float *__restrict__ Ws,
+                            const float *__restrict__ Wm, const int *__restrict__ ptr,
+                            const int *__restrict__ col, const float *__restrict__ val,
+                            const float *__restrict__ h, float *dT, float *dz_out, int n)
 {
+    __shared__ float s1[kH * kH], s2[kH * kH];
+    for (int t = threadIdx.x; t < kH * kH; t += blockDim.x) {
+        s1[(t % kH) * kH + t / kH] = Ws[t];
+        s2[(t % kH) * kH + t / kH] = Wm[t];
+    }
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
          i += (gridDim.x * blockDim.x) >> 5) {
-        const float d = diag ? diag[i] : diag_const;
-        float acc = d * in[size_t(i) * kH + lane];
-        const int k0 = ptr[i], k1 = ptr[i + 1];
-        int k = k0;
-        for (; k + 4 <= k1; k += 4) {
-            float w[4], x[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                w[u] = map ? val[map[k + u]] : val[k + u];
-                x[u] = in[size_t(col[k + u]) * kH + lane];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) acc = fmaf(w[u], x[u], acc);
-        }
-        for (; k < k1; k++) acc = fmaf(map ? val[map[k]] : val[k], in[size_t(col[k]) * kH + lane], acc);
-        out[size_t(i) * kH + lane] = acc;
+        const size_t at = size_t(i) * kH + lane;
+        const float t = spmm_row(ptr[i], ptr[i + 1], col, val, nullptr, dz, lane, 0.f);
+        dT[at] = t;
+        const float d = row_times(t, s2, lane, row_times(dz[at], s1, lane, 0.f));
+        dz_out[at] = h[at] > 0.f ? d : 0.f;
     }
 }
+
+// Sums over the warp of kAhead values a lane each, together: nine shuffles
+// instead of five a value.  Lane l gets the total of value sum_slot(l).
+__device__ __forceinline__ float warp_sums(float (&v)[kAhead], int lane)
+{
+    static_assert(kAhead == 8, "three halvings, then two plain steps");
+    float a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float keep = lane & 16 ? v[4 + i] : v[i], give = lane & 16 ? v[i] : v[4 + i];
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const float keep = lane & 8 ? a[2 + i] : a[i], give = lane & 8 ? a[i] : a[2 + i];
+        b[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+    float t = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[0] : b[1], 4);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    return t;
+}
+__device__ __forceinline__ int sum_slot(int lane) { return lane >> 2; }
 
 // Output head: g_ii = softplus(h_i.w_d + c_d); g_ij = ahat_ij (sum_c w_e h_i h_j + c_e).
 __global__ void k_head(const float *__restrict__ h, const int *__restrict__ lptr,
@@ -144,9 +214,14 @@ __global__ void k_head(const float *__restrict__ h, const int *__restrict__ lptr
             gdiag[i] = softplus_f(u);
         }
         const float hw = hi * we;
-        for (int k = lptr[i]; k < lptr[i + 1]; k++) {
-            const float v = warp_sum_f(hw * h[size_t(lcol[k]) * kH + lane]) + ce;
-            if (lane == 0) goff[k] = lval[k] * v;
+        const int k0 = lptr[i], k1 = lptr[i + 1];
+        for (int k = k0; k < k1; k += kAhead) {
+            float v[kAhead];
+#pragma unroll
+            for (int e = 0; e < kAhead; e++) v[e] = k + e < k1 ? hw * h[size_t(lcol[k + e]) * kH + lane] : 0.f;
+            const float t = warp_sums(v, lane) + ce;
+            const int kk = k + sum_slot(lane);
+            if ((lane & 3) == 0 && kk < k1) goff[kk] = lval[kk] * t;
         }
     }
 }
@@ -174,10 +249,13 @@ __global__ void k_colsum_prod(const float *__restrict__ a, const float *__restri
 }
 
 // part[blk][k*32 + c] = sum over this CTA's rows of a[i,k] * b[i,c]
-// (a: n x ka, ka <= 32) and part[blk][ka*32 + c] = sum b[i,c].
-__global__ void k_outer(const float *__restrict__ a, int ka, const float *__restrict__ b, int n,
-                        float *part)
+// (a: n x ka, ka <= 32) and part[blk][32*32 + c] = sum b[i,c]; with two rows of
+// CTAs (gridDim.y = 2) the second does the same for b2, into the partials after.
+__global__ void k_outer(const float *__restrict__ a, int ka, const float *__restrict__ b1,
+                        const float *__restrict__ b2, int n, float *part)
 {
+    const float *__restrict__ b = blockIdx.y ? b2 : b1;
+    part += size_t(blockIdx.y) * gridDim.x * (kH + 1) * kH;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float acc[kH + 1];
 #pragma unroll
@@ -204,32 +282,36 @@ __global__ void k_outer(const float *__restrict__ a, int ka, const float *__rest
     }
 }
 
-// out[t] = sum_blk part[blk][t] for t < count (fixed order); optional add-to.
-__global__ void k_reduce_parts(const float *__restrict__ part, int nparts, int stride, int count,
-                               float *out, int accumulate)
+// Sums over the CTAs' partials in a fixed order: out1[t] = sum_blk part[blk][t]
+// for t < count1, out2[t] = sum_blk part[blk][off2 + t] for t < count2.  A CTA
+// takes 32 values: each warp an eighth of the partials, its loads independent,
+// then the eighths in order.  (A thread a value was a chain of 256 loads: about
+// 30 us a reduction, 17 of them in a step.)
+__global__ void __launch_bounds__(256) k_reduce_parts(const float *__restrict__ part, int nparts, int stride, int count1,
+                                                      float *out1, int off2, int count2, float *out2)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-        float v = 0.f;
-        for (int p = 0; p < nparts; p++) v += part[size_t(p) * stride + t];
-        out[t] = accumulate ? out[t] + v : v;
+    __shared__ float s[8][kH];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = int(blockIdx.x) * kH + lane;
+    float v = 0.f;
+    if (t < count1 + count2) {
+        const float *p = part + (t < count1 ? t : off2 + t - count1);
+        const int each = (nparts + 7) / 8, p1 = min(nparts, (warp + 1) * each);
+#pragma unroll 8
+        for (int i = warp * each; i < p1; i++) v += p[size_t(i) * stride];
+    }
+    s[warp][lane] = v;
+    __syncthreads();
+    if (warp == 0 && t < count1 + count2) {
+        float r = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) r += s[w][lane];
+        if (t < count1) out1[t] = r;
+        else out2[t - count1] = r;
     }
 }
 
 // --------------------------------------------------------- loss / probes
-// out[i,c] = scale[c] * (a[i,c] - b[i,c])  (b optional), scale optional.
-__global__ void k_axpy_cols(const float *__restrict__ a, const float *__restrict__ b,
-                            const float *__restrict__ scale, float *out, int n)
-{
-    const size_t total = size_t(n) * kH;
-    for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < total;
-         t += size_t(gridDim.x) * blockDim.x) {
-        const int c = int(t % kH);
-        float v = a[t] - (b ? b[t] : 0.f);
-        if (scale) v *= scale[c];
-        out[t] = v;
-    }
-}
-
 // dG on the lower pattern: dGoff[e] = sum_k T[i,k] GU[j,k] + GT[i,k] R[j,k];
 // dGdiag[i] the same with j = i.
 __global__ void k_dG(const float *__restrict__ T, const float *__restrict__ GU,
@@ -243,16 +325,26 @@ __global__ void k_dG(const float *__restrict__ T, const float *__restrict__ GU,
         const float ti = T[size_t(i) * kH + lane], gti = GT[size_t(i) * kH + lane];
         const float dd = warp_sum_f(ti * GU[size_t(i) * kH + lane] + gti * R[size_t(i) * kH + lane]);
         if (lane == 0) dGdiag[i] = dd;
-        for (int k = lptr[i]; k < lptr[i + 1]; k++) {
-            const size_t j = size_t(lcol[k]) * kH + lane;
-            const float v = warp_sum_f(ti * GU[j] + gti * R[j]);
-            if (lane == 0) dGoff[k] = v;
+        const int k0 = lptr[i], k1 = lptr[i + 1];
+        for (int k = k0; k < k1; k += kAhead) {
+            float v[kAhead];
+#pragma unroll
+            for (int e = 0; e < kAhead; e++) {
+                v[e] = 0.f;
+                if (k + e < k1) {
+                    const size_t j = size_t(lcol[k + e]) * kH + lane;
+                    v[e] = ti * GU[j] + gti * R[j];
+                }
+            }
+            const float t = warp_sums(v, lane);
+            const int kk = k + sum_slot(lane);
+            if ((lane & 3) == 0 && kk < k1) dGoff[kk] = t;
         }
     }
 }
 
 // Head backward, pass 1 (rows i over their lower entries): dh_i, dv, and per
-// CTA partials of dw_e (32), dc_e, dw_d (32), dc_d.
+// CTA partials of dw_d (32), dc_d, dw_e (32), dc_e.
 __global__ void k_head_bwd_rows(const float *__restrict__ h, const int *__restrict__ lptr,
                                 const int *__restrict__ lcol, const float *__restrict__ lval,
                                 const float *__restrict__ P, const float *__restrict__ dGoff,
@@ -269,22 +361,35 @@ __global__ void k_head_bwd_rows(const float *__restrict__ h, const int *__restri
         float dhi = du * wd;
         awd = fmaf(du, hi, awd);
         acd += (lane == 0) ? du : 0.f;
-        for (int k = lptr[i]; k < lptr[i + 1]; k++) {
-            const float d = dGoff[k] * lval[k];
-            const float hj = h[size_t(lcol[k]) * kH + lane];
-            dhi = fmaf(d * we, hj, dhi);
-            awe = fmaf(d, hi * hj, awe);
-            ace += (lane == 0) ? d : 0.f;
-            if (lane == 0) dv[k] = d;
+        const int k0 = lptr[i], k1 = lptr[i + 1];
+        for (int k = k0; k < k1; k += kAhead) {
+            float d[kAhead], hj[kAhead];
+#pragma unroll
+            for (int e = 0; e < kAhead; e++) {
+                if (k + e < k1) {
+                    d[e] = dGoff[k + e] * lval[k + e];
+                    hj[e] = h[size_t(lcol[k + e]) * kH + lane];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < kAhead; e++) {
+                if (k + e < k1) {
+                    dhi = fmaf(d[e] * we, hj[e], dhi);
+                    awe = fmaf(d[e], hi * hj[e], awe);
+                    ace += (lane == 0) ? d[e] : 0.f;
+                }
+            }
+            if (lane < kAhead && k + lane < k1) dv[k + lane] = dGoff[k + lane] * lval[k + lane];
         }
         dh[size_t(i) * kH + lane] = dhi;
     }
+    // in the parameters' order: w_d, c_d, w_e, c_e
     __shared__ float s[8][66];
-    s[warp][lane] = awe;
-    s[warp][32 + lane] = awd;
+    s[warp][lane] = awd;
+    s[warp][33 + lane] = awe;
     if (lane == 0) {
-        s[warp][64] = ace;
-        s[warp][65] = acd;
+        s[warp][32] = acd;
+        s[warp][65] = ace;
     }
     __syncthreads();
     for (int t = threadIdx.x; t < 66; t += blockDim.x) {
@@ -295,30 +400,35 @@ __global__ void k_head_bwd_rows(const float *__restrict__ h, const int *__restri
 }
 
 // Head backward, pass 2 (rows j over the transposed lower pattern): adds
-// sum_{i>j} dv_ij w_e h_i into dh_j.
+// sum_{i>j} dv_ij w_e h_i to dh_j and masks it by the last layer's relu:
+// dz = dh where h > 0.
 __global__ void k_head_bwd_cols(const float *__restrict__ h, const int *__restrict__ uptr,
                                 const int *__restrict__ urow, const int *__restrict__ umap,
                                 const float *__restrict__ P, const float *__restrict__ dv,
-                                float *dh, int n)
+                                const float *__restrict__ dh, float *dz, int n)
 {
     const int lane = threadIdx.x & 31;
     const float we = P[kOffWe + lane];
     for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < n;
          j += (gridDim.x * blockDim.x) >> 5) {
-        float acc = dh[size_t(j) * kH + lane];
-        for (int k = uptr[j]; k < uptr[j + 1]; k++)
-            acc = fmaf(dv[umap[k]] * we, h[size_t(urow[k]) * kH + lane], acc);
-        dh[size_t(j) * kH + lane] = acc;
+        const size_t at = size_t(j) * kH + lane;
+        float acc = dh[at];
+        const int k0 = uptr[j], k1 = uptr[j + 1];
+        for (int k = k0; k < k1; k += kAhead) {
+            float d[kAhead], x[kAhead];
+#pragma unroll
+            for (int e = 0; e < kAhead; e++) {
+                if (k + e < k1) {
+                    d[e] = dv[umap[k + e]];
+                    x[e] = h[size_t(urow[k + e]) * kH + lane];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < kAhead; e++)
+                if (k + e < k1) acc = fmaf(d[e] * we, x[e], acc);
+        }
+        dz[at] = h[at] > 0.f ? acc : 0.f;
     }
-}
-
-// dz = dh * (h > 0)
-__global__ void k_relu_bwd(const float *__restrict__ dh, const float *__restrict__ h, float *dz,
-                           size_t total)
-{
-    for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < total;
-         t += size_t(gridDim.x) * blockDim.x)
-        dz[t] = h[t] > 0.f ? dh[t] : 0.f;
 }
 
 // Adam on the flat parameter vector.
@@ -459,7 +569,7 @@ struct cgb_gnn {
     int sms = 148;
     cudaStream_t stream = nullptr;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;  // params, grad, Adam moments
-    float *part = nullptr;   // kRedBlocks x 33 x 32
+    float *part = nullptr;   // 2 x kRedBlocks x 33 x 32
     float *colv = nullptr;   // small per-column vectors (8 x 32)
     float *loss = nullptr;
     int adam_t = 0;
@@ -467,7 +577,9 @@ struct cgb_gnn {
 
 namespace {
 
-int grid_rows(const cgb_gnn *m, int n) { return std::max(1, std::min(8 * m->sms, (n + 7) / 8)); }
+// CTAs of a warp-a-row kernel: a row a warp up to 64 CTAs an SM, so that the
+// SMs even out uneven rows.
+int grid_rows(const cgb_gnn *m, int n) { return std::max(1, std::min(64 * m->sms, (n + 7) / 8)); }
 
 void free_graph(cgb_gnn_graph *g)
 {
@@ -514,46 +626,54 @@ int forward(cgb_gnn *m, cgb_gnn_graph *g)
 {
     const int n = g->n, gr = grid_rows(m, n);
     const float *P = m->P;
-    k_dense<<<gr, 256, 0, m->stream>>>(g->X, kF, P + kOffWin, P + kOffBin, nullptr, g->Hs[0], n, 1);
-    for (int l = 0; l < kL; l++) {
-        const float *Ws = P + kOffLayer + l * kLayerSize;
-        const float *Wm = Ws + kH * kH;
-        const float *b = Wm + kH * kH;
-        k_dense<<<gr, 256, 0, m->stream>>>(g->Hs[l], kH, Wm, nullptr, nullptr, g->T, n, 0);
-        k_spmm<<<gr, 256, 0, m->stream>>>(g->off_ptr, g->off_col, g->off_val, nullptr, nullptr, 0.f,
-                                         g->T, g->U, n);
-        k_dense<<<gr, 256, 0, m->stream>>>(g->Hs[l], kH, Ws, b, g->U, g->Hs[l + 1], n, 1);
-    }
+    auto Ws = [&](int l) { return P + kOffLayer + l * kLayerSize; };
+    k_dense<<<gr, 256, 0, m->stream>>>(g->X, kF, P + kOffWin, P + kOffBin, g->Hs[0], n, 1);
+    k_dense<<<gr, 256, 0, m->stream>>>(g->Hs[0], kH, Ws(0) + kH * kH, nullptr, g->T, n, 0);
+    float *T[2] = {g->T, g->U};
+    for (int l = 0; l < kL; l++)
+        k_layer<<<gr, 256, 0, m->stream>>>(g->Hs[l], T[l & 1], Ws(l), Ws(l) + 2 * kH * kH, g->off_ptr, g->off_col,
+                                          g->off_val, l + 1 < kL ? Ws(l + 1) + kH * kH : nullptr, g->Hs[l + 1],
+                                          T[(l + 1) & 1], n);
     k_head<<<gr, 256, 0, m->stream>>>(g->Hs[kL], g->low_ptr, g->low_col, g->low_val, P, g->goff,
                                      g->gdiag, g->ud, n);
     GNN_TRY(cudaGetLastError());
     return CGB_OK;
 }
 
-// Y = Ahat X = diag(Ahat) X + Aoff X.
-void ahat_mm(cgb_gnn *m, cgb_gnn_graph *g, const float *X, float *Y)
+// Y = cscale (Ahat X - sub), Ahat X = diag(Ahat) X + Aoff X (sub, cscale may
+// be null).
+void ahat_mm(cgb_gnn *m, cgb_gnn_graph *g, const float *X, float *Y, const float *sub = nullptr,
+             const float *cscale = nullptr)
 {
     k_spmm<<<grid_rows(m, g->n), 256, 0, m->stream>>>(g->off_ptr, g->off_col, g->off_val, nullptr,
-                                                     g->adiag, 0.f, X, Y, g->n);
+                                                     g->adiag, X, sub, cscale, Y, g->n);
 }
 // Y = G X (lower pattern + diagonal)
 void g_mm(cgb_gnn *m, cgb_gnn_graph *g, const float *X, float *Y)
 {
     k_spmm<<<grid_rows(m, g->n), 256, 0, m->stream>>>(g->low_ptr, g->low_col, g->goff, nullptr,
-                                                     g->gdiag, 0.f, X, Y, g->n);
+                                                     g->gdiag, X, nullptr, nullptr, Y, g->n);
 }
 // Y = G^T X (transposed pattern, values through the map)
 void gt_mm(cgb_gnn *m, cgb_gnn_graph *g, const float *X, float *Y)
 {
     k_spmm<<<grid_rows(m, g->n), 256, 0, m->stream>>>(g->up_ptr, g->up_row, g->goff, g->up_map,
-                                                     g->gdiag, 0.f, X, Y, g->n);
+                                                     g->gdiag, X, nullptr, nullptr, Y, g->n);
+}
+
+// Sums of the partials in m->part (see k_reduce_parts).
+void reduce_parts(cgb_gnn *m, const float *part, int stride, int count1, float *out1, int off2 = 0, int count2 = 0,
+                  float *out2 = nullptr, int nparts = kRedBlocks)
+{
+    k_reduce_parts<<<(count1 + count2 + kH - 1) / kH, 256, 0, m->stream>>>(part, nparts, stride, count1, out1, off2,
+                                                                          count2, out2);
 }
 
 // Column sums of a*b (b null: a*a) into m->colv + 32*slot.
 void colsum(cgb_gnn *m, const float *a, const float *b, int n, int slot)
 {
     k_colsum_prod<<<kRedBlocks, 256, 0, m->stream>>>(a, b, n, m->part);
-    k_reduce_parts<<<1, 32, 0, m->stream>>>(m->part, kRedBlocks, kH, kH, m->colv + kH * slot, 0);
+    reduce_parts(m, m->part, kH, kH, m->colv + kH * slot);
 }
 
 // Probes: 32 columns of R.  `cg_steps` = 0: normal random vectors; else the
@@ -590,32 +710,27 @@ int make_probes(cgb_gnn *m, cgb_gnn_graph *g, unsigned seed, int cg_steps)
 int loss_grad(cgb_gnn *m, cgb_gnn_graph *g)
 {
     const int n = g->n, gr = grid_rows(m, n);
-    const size_t total = size_t(n) * kH;
     int st = forward(m, g);
     if (st) return st;
     float *rn2 = m->colv + 5 * kH, *wn2 = m->colv + 6 * kH, *coef = m->colv + 7 * kH;
     colsum(m, g->R, nullptr, n, 5);
     g_mm(m, g, g->R, g->Tg);           // T = G R
     gt_mm(m, g, g->Tg, g->Ug);         // U = G^T T
-    ahat_mm(m, g, g->Ug, g->W);        // W = Ahat U
-    k_axpy_cols<<<gr, 256, 0, m->stream>>>(g->W, g->R, nullptr, g->W, n);  // W -= R
+    ahat_mm(m, g, g->Ug, g->W, g->R);  // W = Ahat U - R
     colsum(m, g->W, nullptr, n, 6);
     k_loss_coef<<<1, 32, 0, m->stream>>>(rn2, wn2, coef, m->loss);
-    ahat_mm(m, g, g->W, g->GU);        // GU = Ahat W, scaled per column
-    k_axpy_cols<<<gr, 256, 0, m->stream>>>(g->GU, nullptr, coef, g->GU, n);
+    ahat_mm(m, g, g->W, g->GU, nullptr, coef);  // GU = Ahat W, scaled per column
     g_mm(m, g, g->GU, g->GT);          // GT = G GU
     k_dG<<<gr, 256, 0, m->stream>>>(g->Tg, g->GU, g->GT, g->R, g->low_ptr, g->low_col, g->dGoff,
                                    g->dGdiag, n);
     // head backward
-    k_head_bwd_rows<<<kRedBlocks, 256, 0, m->stream>>>(g->Hs[kL], g->low_ptr, g->low_col,
+    k_head_bwd_rows<<<kHeadBlocks, 256, 0, m->stream>>>(g->Hs[kL], g->low_ptr, g->low_col,
                                                       g->low_val, m->P, g->dGoff, g->dGdiag, g->ud,
                                                       g->dv, g->dh, m->part, n);
-    k_reduce_parts<<<1, 96, 0, m->stream>>>(m->part, kRedBlocks, 66, 32, m->G + kOffWe, 0);
-    k_reduce_parts<<<1, 96, 0, m->stream>>>(m->part + 32, kRedBlocks, 66, 32, m->G + kOffWd, 0);
-    k_reduce_parts<<<1, 32, 0, m->stream>>>(m->part + 64, kRedBlocks, 66, 1, m->G + kOffCe, 0);
-    k_reduce_parts<<<1, 32, 0, m->stream>>>(m->part + 65, kRedBlocks, 66, 1, m->G + kOffCd, 0);
+    reduce_parts(m, m->part, 66, 66, m->G + kOffWd, 0, 0, nullptr, kHeadBlocks);
+    float *dz = g->dz, *dz_next = g->dh;
     k_head_bwd_cols<<<gr, 256, 0, m->stream>>>(g->Hs[kL], g->up_ptr, g->up_row, g->up_map, m->P,
-                                              g->dv, g->dh, n);
+                                              g->dv, g->dh, dz, n);
     // message-passing layers, last to first
     const int ostride = (kH + 1) * kH;
     for (int l = kL - 1; l >= 0; l--) {
@@ -624,21 +739,15 @@ int loss_grad(cgb_gnn *m, cgb_gnn_graph *g)
         float *gWs = m->G + kOffLayer + l * kLayerSize;
         float *gWm = gWs + kH * kH;
         float *gb = gWm + kH * kH;
-        k_relu_bwd<<<gr, 256, 0, m->stream>>>(g->dh, g->Hs[l + 1], g->dz, total);
-        k_outer<<<kRedBlocks, 256, 0, m->stream>>>(g->Hs[l], kH, g->dz, n, m->part);
-        k_reduce_parts<<<8, 128, 0, m->stream>>>(m->part, kRedBlocks, ostride, kH * kH, gWs, 0);
-        k_reduce_parts<<<1, 32, 0, m->stream>>>(m->part + kH * kH, kRedBlocks, ostride, kH, gb, 0);
-        k_spmm<<<gr, 256, 0, m->stream>>>(g->off_ptr, g->off_col, g->off_val, nullptr, nullptr, 0.f,
-                                         g->dz, g->dT, n);  // dT = Aoff dz
-        k_outer<<<kRedBlocks, 256, 0, m->stream>>>(g->Hs[l], kH, g->dT, n, m->part);
-        k_reduce_parts<<<8, 128, 0, m->stream>>>(m->part, kRedBlocks, ostride, kH * kH, gWm, 0);
-        k_dense_t2<<<gr, 256, 0, m->stream>>>(g->dz, Ws, g->dT, Wm, g->dh, n);
+        k_layer_bwd<<<gr, 256, 0, m->stream>>>(dz, Ws, Wm, g->off_ptr, g->off_col, g->off_val, g->Hs[l], g->dT,
+                                              dz_next, n);
+        k_outer<<<dim3(kRedBlocks, 2), 256, 0, m->stream>>>(g->Hs[l], kH, dz, g->dT, n, m->part);
+        reduce_parts(m, m->part, ostride, kH * kH, gWs, kH * kH, kH, gb);
+        reduce_parts(m, m->part + size_t(kRedBlocks) * ostride, ostride, kH * kH, gWm);
+        std::swap(dz, dz_next);
     }
-    k_relu_bwd<<<gr, 256, 0, m->stream>>>(g->dh, g->Hs[0], g->dz, total);
-    k_outer<<<kRedBlocks, 256, 0, m->stream>>>(g->X, kF, g->dz, n, m->part);
-    k_reduce_parts<<<1, 128, 0, m->stream>>>(m->part, kRedBlocks, ostride, kF * kH, m->G + kOffWin, 0);
-    k_reduce_parts<<<1, 32, 0, m->stream>>>(m->part + kH * kH, kRedBlocks, ostride, kH,
-                                           m->G + kOffBin, 0);
+    k_outer<<<kRedBlocks, 256, 0, m->stream>>>(g->X, kF, dz, nullptr, n, m->part);
+    reduce_parts(m, m->part, ostride, kF * kH, m->G + kOffWin, kH * kH, kH, m->G + kOffBin);
     GNN_TRY(cudaGetLastError());
     return CGB_OK;
 }
@@ -666,7 +775,7 @@ int cgb_gnn_create(int device, unsigned seed, cgb_gnn **out)
     m->sms = prop.multiProcessorCount;
     if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
         galloc(&m->P, kNumParams) || galloc(&m->G, kNumParams) || galloc(&m->M, kNumParams) ||
-        galloc(&m->V, kNumParams) || galloc(&m->part, size_t(kRedBlocks) * (kH + 1) * kH) ||
+        galloc(&m->V, kNumParams) || galloc(&m->part, 2 * size_t(kRedBlocks) * (kH + 1) * kH) ||
         galloc(&m->colv, 8 * kH) || galloc(&m->loss, 1)) {
         cgb_gnn_destroy(m);
         return set_error(CGB_ERR_NOMEM, "model device allocation failed");

@@ -76,6 +76,33 @@ def test_gnn_gradient_matches_oracle(cgb, small_case):
     assert not bad, bad
 
 
+@pytest.mark.parametrize("n,half", [(3, 1), (31, 2), (33, 3), (257, 4), (1001, 9)])
+def test_gnn_gradient_by_row_length(cgb, n, half):
+    """Loss and gradient on rings with 2 x `half` neighbours a row: fewer than,
+    exactly and more than the 8 gathers in flight of the sparse products (the
+    lower pattern's rows have 0 to 2 x half), n below and beside a block of 8
+    rows.  The bounds are those of test_gnn_gradient_matches_oracle."""
+    import gnn_oracle as go
+    cols = (np.arange(n)[:, None] + np.arange(-half, half + 1)) % n
+    cols.sort(axis=1)
+    i = np.arange(n)[:, None]
+    dist = np.minimum((cols - i) % n, (i - cols) % n)
+    a = np.where(dist == 0, -2.0 * half - 1.0 - 0.1 * (i % 3), np.cos(0.7 * dist + 0.1 * ((i + cols) % 5)))
+    rs = np.arange(0, n * (2 * half + 1) + 1, 2 * half + 1, dtype=np.int32)
+    ci, a = cols.astype(np.int32).ravel(), a.ravel()
+    model = cgb.Gnn(seed=11)
+    rng = np.random.default_rng(5)
+    model.params = model.params + rng.normal(0, 0.05, model.n_params).astype(np.float32)
+    probes = rng.normal(size=(n, 32)).astype(np.float32)
+    with model.graph(rs, ci, a) as g:
+        loss, grad = model.loss_grad(g, probes=probes)
+    Lref, gref, _ = go.loss_and_grad(go.unflatten(model.params), go.Graph(rs, ci, a), probes.astype(np.float64))
+    assert abs(loss - Lref) <= 1e-4 * abs(Lref)
+    errs = group_errors(go, grad, gref)
+    bad = {k: v for k, v in errs.items() if v > 2e-3}
+    assert not bad, bad
+
+
 def test_gnn_generated_probes_and_training_lowers_loss(cgb):
     model = cgb.Gnn(seed=3)
     mats = [cgb.makea(2000, 7, 0.1, 10.0, s) for s in (1000003.0, 1000005.0)]
