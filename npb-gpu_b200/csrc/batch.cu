@@ -32,15 +32,12 @@
 //          preconditioned iteration stalls (|r|^2 not halved in four steps,
 //          or r.y <= 0) continues as plain CG; a system showing p.Ap >= 0 is
 //          re-solved with the FP64 reference algorithm, as in the mixed mode.
-// The matrices are stored as slices of 32 rows sorted by length, a lane a row
-// (plan_slices); the factors' lanes per row are a per-system choice (the
-// autotuner's, by row length).
+// Lanes per row are a per-system choice (the autotuner's, by row length).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <functional>
 #include <new>
 #include <numeric>
 #include <vector>
@@ -56,7 +53,6 @@ namespace batch {
 
 constexpr int kBatchMaxN = 27000;  // rows of the largest system (shared p: 8 bytes a row)
 constexpr int kReferenceCgitmax = 25;  // cg.cu's cgitmax: the FP64 re-solve of a mixed failure
-constexpr int kLongRow = 1 << 30;      // flag of a row that is a slice of its own
 constexpr int kMaxTeam = 8;            // CTAs that may share one system
 constexpr int kTeamValues = 16;        // values one team reduction can carry
 constexpr int kSyncStride = 32;        // words between barrier counters (128-byte lines)
@@ -65,12 +61,11 @@ static_assert(kTeamValues >= kGramValues, "team reductions must carry the Gram v
 
 struct SysDesc {
     int n;
+    int lanes;           // lanes per row (2, 4, 8, 16, 32)
     int team;            // CTAs that solve the system together (1, 2, 4 or 8)
     int flanes;          // lanes per row of the preconditioner's factor products
-    int slices;          // slices of its rows
     long long row_off;   // into rowstr_all (n+1 entries)
-    long long slice_off; // into slice_rows (32 a slice) and slice_start
-    long long entry_off; // into the slices' entries (a, a32, col)
+    long long nnz_off;   // into colidx_all / a_all
     long long vec_off;   // into the vector arrays (n+8 entries)
     long long f_row_off; // into the factor row pointers (F and F^T: n+1 entries each)
     long long f_off;     // into the factor entries (F and F^T: the same count)
@@ -86,17 +81,9 @@ struct BatchArgs {
     int nsys;
     const SysDesc *__restrict__ sys;
     const int *__restrict__ rowstr;
-    // the matrices as slices of 32 rows, longest first: slice_rows holds a
-    // lane's row (-1: none) and its number of entries, slice_start the slice's
-    // first entry (from entry_off), and lane l's entry k lies at start +
-    // 64 (k / 2) + 2 l + k % 2.  A row much longer than the system's mean has a
-    // slice to itself, its pairs dealt to the lanes in turn (kLongRow is set in
-    // the row, and the lanes' sums are added).
-    const int2 *__restrict__ slice_rows;
-    const long long *__restrict__ slice_start;
+    const int *__restrict__ colidx;
     const double *__restrict__ a;
     const float *__restrict__ a32;
-    const unsigned short *__restrict__ col;
     double *x, *z, *r, *q;
     unsigned *queue;
     int mode;            // 0 fixed, 1 mixed (the launch's kernel)
@@ -274,144 +261,80 @@ __device__ __forceinline__ bool team_sum_multi(const TeamMem &M, Team &T, const 
     return true;
 }
 
-// Rows [lo, hi) of this thread, kAhead at a time: `load` for each, then `use`
-// for each in order.  A row at a time, every row is a trip to L2 or HBM (20 of
-// them a pass for the largest systems at 1024 threads).
-constexpr int kAhead = 4;
-template <typename V, typename Load, typename Use>
-__device__ __forceinline__ void for_rows(int lo, int hi, Load load, Use use)
-{
-    int j = lo + int(threadIdx.x);
-    const int step = int(blockDim.x);
-    for (; j + (kAhead - 1) * step < hi; j += kAhead * step) {
-        V v[kAhead];
-#pragma unroll
-        for (int u = 0; u < kAhead; u++) v[u] = load(j + u * step);
-#pragma unroll
-        for (int u = 0; u < kAhead; u++) use(j + u * step, v[u]);
-    }
-    for (; j < hi; j += step) use(j, load(j));
-}
-
 // After a team barrier that followed the members' writes of their rows of
 // p to pg: the other members' rows into this CTA's shared copy.
 __device__ __forceinline__ void team_gather_p(const Team &T, const double *pg, double *p, int n)
 {
     if (T.size == 1) return;
-    auto load = [&](int j) { return __ldcg(pg + j); };
-    auto use = [&](int j, double v) { p[j] = v; };
-    for_rows<double>(0, T.lo, load, use);
-    for_rows<double>(T.hi, n, load, use);
+    for (int j = threadIdx.x; j < T.lo; j += blockDim.x) p[j] = __ldcg(pg + j);
+    for (int j = T.hi + threadIdx.x; j < n; j += blockDim.x) p[j] = __ldcg(pg + j);
     __syncthreads();
 }
 
-// q[row] = (A v)[row] for the rows of the team's slices that are this CTA's
-// (every team-size-th of the warps' slices); v in shared memory (FP64, or VS)
-// or, v_gl, in global memory.  `cg`: a team's -- vectors in global memory are
-// read through L2, since other members' rows may have been written since this
-// SM last cached them, and so is q afterwards (q_at).  Products in FP64, or
-// (F32) in FP32 values summed in FP64 after every kU pairs; returns this
-// thread's share of sum_row dv[row] q[row] (dv: shared p, a global vector with
-// dv_cg, or null).
-//
-// A lane owns a row, so a warp streams 32 rows with kU independent pairs of
-// entries in flight a lane (16-byte values, 4-byte columns), where a row a warp
-// spent its time on a row's pointers, two bursts of loads and a reduction: 128
-// systems, FP64, 1024 threads: 146 ms a row a warp.
+// q[j] = (A v)[j] for rows [lo, hi) of the system with S.lanes lanes per
+// row; v in shared memory (FP64) or, v_gl, global memory (v_gl_shared: a
+// team's vector, read through L2, since other members' rows may have been
+// written since this SM last cached them); products in FP64 or (F32) in FP32 with FP32 row sums; returns this
+// thread's share of sum_j dv[j] q[j] (dv: shared p or null).  The lane count
+// is a run-time value: one instance of the solver serves every system (an
+// instance per lane count inlined under one switch needed 128 registers a
+// thread and spilled; one needs about 84).
 template <typename T>
 struct NoDeduce {
     using type = T;
 };
 
 template <bool F32, int kU, typename VS = double>
-__device__ __forceinline__ double sys_spmv(const BatchArgs &B, const SysDesc &S, const Team &T,
-                                           const typename NoDeduce<VS>::type *v_sh, const double *v_gl, double *q,
-                                           const double *dv, bool cg, bool dv_cg = false)
+__device__ __forceinline__ double sys_spmv(const BatchArgs &B, const SysDesc &S, int lo, int hi,
+                                           const typename NoDeduce<VS>::type *v_sh,
+                                           const double *v_gl, double *q,
+                                           const double *dv_sh, bool v_gl_shared = false)
 {
-    const int2 *rows = B.slice_rows + S.slice_off * 32;
-    const long long *starts = B.slice_start + S.slice_off;
-    const double *a = B.a + S.entry_off;
-    const float *a32 = B.a32 + S.entry_off;
-    const unsigned short *col = B.col + S.entry_off;
-    const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) * T.size;
-    const int w = T.member * int(blockDim.x >> 5) + int(threadIdx.x >> 5);
-    // slice i of this warp, in boustrophedon order so that the warps' sums of
-    // lengths stay close
-    auto slice = [&](int i, int2 &mine, long long &start) {
-        const int s = i * nw + ((i & 1) ? nw - 1 - w : w);
-        mine = s < S.slices ? __ldg(rows + size_t(s) * 32 + lane) : make_int2(-1, 0);
-        start = s < S.slices ? __ldg(starts + s) + 2 * lane : 0;
-    };
-    auto vec = [&](int c) { return v_sh ? double(v_sh[c]) : (cg ? __ldcg(v_gl + c) : v_gl[c]); };
+    const int *rowstr = B.rowstr + S.row_off;
+    const int *colidx = B.colidx + S.nnz_off;
+    const double *a = B.a + S.nnz_off;
+    const float *a32 = B.a32 ? B.a32 + S.nnz_off : nullptr;
+    const int LPR = S.lanes;
+    const int lane = threadIdx.x & (LPR - 1), grp = threadIdx.x / LPR, ngrp = blockDim.x / LPR;
+    const unsigned mask =
+        LPR == 32 ? 0xffffffffu : (((1u << LPR) - 1u) << ((threadIdx.x & 31) & ~(LPR - 1)));
     double dacc = 0.0;
-    int2 mine, next;
-    long long start, next_start;
-    slice(0, mine, start);
-    for (int i = 0; i * nw < S.slices; i++) {
-        slice(i + 1, next, next_start);
-        const int len = mine.y;
-        double sx = 0.0, sy = 0.0;
-        for (int k = 0; k < len; k += 2 * kU) {
-            ushort2 c[kU];
-            if constexpr (F32) {
-                float2 v[kU];
+    for (int row = lo + grp; row < hi; row += ngrp) {
+        const int k0 = rowstr[row], k1 = rowstr[row + 1];
+        double s64 = 0.0;
+        float s32 = 0.f;
+        for (int k = k0 + lane; k < k1; k += kU * LPR) {
+            int c[kU];
+            double av[kU];
+            float af[kU];
 #pragma unroll
-                for (int u = 0; u < kU; u++) {
-                    if (k + 2 * u < len) {
-                        v[u] = __ldcs(reinterpret_cast<const float2 *>(a32 + start + 32 * (k + 2 * u)));
-                        c[u] = __ldcs(reinterpret_cast<const ushort2 *>(col + start + 32 * (k + 2 * u)));
-                    }
+            for (int u = 0; u < kU; u++) {
+                const int kk = k + u * LPR;
+                if (kk < k1) {
+                    c[u] = __ldcs(colidx + kk);
+                    if (F32) af[u] = __ldcs(a32 + kk);
+                    else av[u] = __ldcs(a + kk);
                 }
-                float fx = 0.f, fy = 0.f;
+            }
 #pragma unroll
-                for (int u = 0; u < kU; u++) {
-                    if (k + 2 * u < len) fx = fmaf(v[u].x, float(vec(c[u].x)), fx);
-                    if (k + 2 * u + 1 < len) fy = fmaf(v[u].y, float(vec(c[u].y)), fy);
-                }
-                sx += double(fx);
-                sy += double(fy);
-            } else {
-                double2 v[kU];
-#pragma unroll
-                for (int u = 0; u < kU; u++) {
-                    if (k + 2 * u < len) {
-                        v[u] = __ldcs(reinterpret_cast<const double2 *>(a + start + 32 * (k + 2 * u)));
-                        c[u] = __ldcs(reinterpret_cast<const ushort2 *>(col + start + 32 * (k + 2 * u)));
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kU; u++) {
-                    if (k + 2 * u < len) sx = fma(v[u].x, vec(c[u].x), sx);
-                    if (k + 2 * u + 1 < len) sy = fma(v[u].y, vec(c[u].y), sy);
+            for (int u = 0; u < kU; u++) {
+                if (k + u * LPR < k1) {
+                    const double pv = v_sh ? double(v_sh[c[u]])
+                                           : (v_gl_shared ? __ldcg(v_gl + c[u]) : v_gl[c[u]]);
+                    if (F32) s32 = fmaf(af[u], float(pv), s32);
+                    else s64 = fma(av[u], pv, s64);
                 }
             }
         }
-        double sum = sx + sy;
-        int row = mine.x;
-        if (__any_sync(0xffffffffu, row >= kLongRow)) {
-            sum = warp_sum(sum);
-            row = lane == 0 ? row - kLongRow : -1;
+        double s;
+        if (F32) s = double(group_sum_f_rt(s32, mask, LPR));
+        else s = group_sum_rt(s64, mask, LPR);
+        if (lane == 0) {
+            q[row] = s;
+            if (dv_sh) dacc = fma(dv_sh[row], s, dacc);
         }
-        if (row >= 0) {
-            q[row] = sum;
-            if (dv) dacc = fma(dv_cg ? __ldcg(dv + row) : dv[row], sum, dacc);
-        }
-        mine = next;
-        start = next_start;
     }
     return dacc;
-}
-
-// Row j of the product last written to q, which another member may have
-// formed (after a team barrier).
-__device__ __forceinline__ double q_at(const double *q, int j, bool team) { return team ? __ldcg(q + j) : q[j]; }
-
-// After a product that no team sum follows: every row of q is written.
-__device__ __forceinline__ bool product_ready(const BatchArgs &B, const Team &T, bool team)
-{
-    if (team) return team_barrier(team_mem(B, T.id), T);
-    __syncthreads();
-    return true;
 }
 
 struct GalerkinIn {
@@ -586,11 +509,11 @@ __device__ int solve_system(const BatchArgs &B, const SysDesc &S, Team &T, int c
                 if (refresh) {
                     // r = x - A z (FP64 matrix; every member's z rows were
                     // published by the last team sum), restart p = r
-                    sys_spmv<false, kU>(B, S, T, nullptr, z, q, nullptr, team);
-                    if (!product_ready(B, T, team)) return kSolveAborted;
+                    sys_spmv<false, kU>(B, S, lo, hi, nullptr, z, q, nullptr, team);
+                    __syncthreads();
                     acc = 0.0;
                     for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
-                        const double rv = x[j] - q_at(q, j, team);
+                        const double rv = x[j] - q[j];
                         r[j] = rv;
                         p[j] = rv;
                         if (team) pg[j] = rv;
@@ -604,35 +527,28 @@ __device__ int solve_system(const BatchArgs &B, const SysDesc &S, Team &T, int c
                     continue;
                 }
             }
-            const double dpart = mixed ? sys_spmv<true, kU>(B, S, T, p, nullptr, q, p, team)
-                                       : sys_spmv<false, kU>(B, S, T, p, nullptr, q, p, team);
+            const double dpart = mixed ? sys_spmv<true, kU>(B, S, lo, hi, p, nullptr, q, p)
+                                       : sys_spmv<false, kU>(B, S, lo, hi, p, nullptr, q, p);
             double d;
             if (!team_sum(B, T, dpart, red, d)) return kSolveAborted;  // barrier: q complete
             if (mixed && !(d < 0.0)) return kSolveGaveUp;  // not negative definite (or NaN)
             const double alpha = rho / d;
             const double rho0 = rho;
             acc = 0.0;
-            struct Row {
-                double z, q, r;
-            };
-            for_rows<Row>(
-                lo, hi, [&](int j) { return Row{z[j], q_at(q, j, team), r[j]}; },
-                [&](int j, Row v) {
-                    z[j] = fma(alpha, p[j], v.z);
-                    const double rv = fma(-alpha, v.q, v.r);
-                    r[j] = rv;
-                    acc = fma(rv, rv, acc);
-                });
+            for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
+                z[j] = fma(alpha, p[j], z[j]);
+                const double rv = fma(-alpha, q[j], r[j]);
+                r[j] = rv;
+                acc = fma(rv, rv, acc);
+            }
             if (!team_sum(B, T, acc, red, rho)) return kSolveAborted;
             if (mixed && !(rho < INFINITY)) return kSolveGaveUp;  // non-finite residual
             const double beta = rho / rho0;
-            for_rows<double>(
-                lo, hi, [&](int j) { return r[j]; },
-                [&](int j, double rv) {
-                    const double pv = fma(beta, p[j], rv);
-                    p[j] = pv;
-                    if (team) pg[j] = pv;
-                });
+            for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
+                const double pv = fma(beta, p[j], r[j]);
+                p[j] = pv;
+                if (team) pg[j] = pv;
+            }
             if (team) {
                 if (!team_barrier(team_mem(B, T.id), T)) return kSolveAborted;
                 team_gather_p(T, pg, p, n);
@@ -649,12 +565,12 @@ __device__ int solve_system(const BatchArgs &B, const SysDesc &S, Team &T, int c
         if (mixed && fresh) {
             for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) q[j] = x[j] - r[j];
         } else {
-            sys_spmv<false, kU>(B, S, T, nullptr, z, q, nullptr, team);
+            sys_spmv<false, kU>(B, S, lo, hi, nullptr, z, q, nullptr, team);
         }
-        if (!product_ready(B, T, team)) return kSolveAborted;
+        __syncthreads();
         double res = 0.0, xz = 0.0, zz = 0.0;
         for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
-            const double xv = x[j], zv = z[j], dv = xv - q_at(q, j, team);
+            const double xv = x[j], zv = z[j], dv = xv - q[j];
             res = fma(dv, dv, res);
             xz = fma(xv, zv, xz);
             zz = fma(zv, zv, zz);
@@ -672,7 +588,7 @@ __device__ int solve_system(const BatchArgs &B, const SysDesc &S, Team &T, int c
             for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
                 const double xn = norm * z[j];
                 B.hx[slot + j] = xn;
-                B.hw[slot + j] = norm * q_at(q, j, team);
+                B.hw[slot + j] = norm * q[j];
                 x[j] = xn;
             }
         } else {
@@ -911,11 +827,11 @@ __device__ int solve_system_pcg(const BatchArgs &B, const SysDesc &S, Team &T, i
             bool restart = refresh;
             if (refresh) {
                 // r' = A z - x with the FP64 matrix (z published by the last team sum)
-                sys_spmv<false, kU>(B, S, T, nullptr, V.z, V.q, nullptr, team);
-                if (!product_ready(B, T, team)) return kSolveAborted;
+                sys_spmv<false, kU>(B, S, lo, hi, nullptr, V.z, V.q, nullptr, team);
+                __syncthreads();
                 acc = 0.0;
                 for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
-                    const double rv = q_at(V.q, j, team) - V.x[j];
+                    const double rv = V.q[j] - V.x[j];
                     V.r[j] = rv;
                     V.v32[j] = float(rv);
                     if (team) V.rg[j] = float(rv);
@@ -930,7 +846,7 @@ __device__ int solve_system_pcg(const BatchArgs &B, const SysDesc &S, Team &T, i
                 if (rr <= stop2) break;
             } else {
                 // q = A32 p32 (FP32 products); p.A'p = -p.q
-                const double dpart = sys_spmv<true, kU, float>(B, S, T, V.p32, nullptr, V.q, V.pg, team, team);
+                const double dpart = sys_spmv<true, kU, float>(B, S, lo, hi, V.p32, nullptr, V.q, V.pg);
                 double d;
                 if (!team_sum(B, T, dpart, red, d)) return kSolveAborted;
                 const double pAp = -d;
@@ -939,7 +855,7 @@ __device__ int solve_system_pcg(const BatchArgs &B, const SysDesc &S, Team &T, i
                 acc = 0.0;
                 for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
                     V.z[j] = fma(alpha, V.pg[j], V.z[j]);
-                    const double rv = fma(alpha, q_at(V.q, j, team), V.r[j]);  // r' -= alpha A'p
+                    const double rv = fma(alpha, V.q[j], V.r[j]);  // r' -= alpha A'p
                     V.r[j] = rv;
                     V.v32[j] = float(rv);
                     if (team) V.rg[j] = float(rv);
@@ -983,12 +899,12 @@ __device__ int solve_system_pcg(const BatchArgs &B, const SysDesc &S, Team &T, i
         if (fresh) {
             for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) V.q[j] = V.x[j] + V.r[j];
         } else {
-            sys_spmv<false, kU>(B, S, T, nullptr, V.z, V.q, nullptr, team);
+            sys_spmv<false, kU>(B, S, lo, hi, nullptr, V.z, V.q, nullptr, team);
         }
-        if (!product_ready(B, T, team)) return kSolveAborted;
+        __syncthreads();
         double res = 0.0, xz = 0.0, zz = 0.0;
         for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
-            const double xv = V.x[j], zv = V.z[j], dv = xv - q_at(V.q, j, team);
+            const double xv = V.x[j], zv = V.z[j], dv = xv - V.q[j];
             res = fma(dv, dv, res);
             xz = fma(xv, zv, xz);
             zz = fma(zv, zv, zz);
@@ -1005,7 +921,7 @@ __device__ int solve_system_pcg(const BatchArgs &B, const SysDesc &S, Team &T, i
             for (int j = lo + threadIdx.x; j < hi; j += blockDim.x) {
                 const double xn = norm * V.z[j];
                 B.hx[slot + j] = xn;
-                B.hw[slot + j] = norm * q_at(V.q, j, team);
+                B.hw[slot + j] = norm * V.q[j];
                 V.x[j] = xn;
             }
         } else {
@@ -1088,28 +1004,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1) batch_kernel(BatchArgs B, cons
     }
 }
 
-// Fills one system's slices from its CSR: a warp a slice (see BatchArgs).
-static __global__ void fill_slices(const int *__restrict__ rowstr, const int *__restrict__ colidx,
-                                   const double *__restrict__ vals, int slices, const int2 *__restrict__ slice_rows,
-                                   const long long *__restrict__ slice_start, double *a, float *a32,
-                                   unsigned short *col)
+static __global__ void to_fp32_batch(const double *__restrict__ in, float *__restrict__ out,
+                                     long long count)
 {
-    const int lane = threadIdx.x & 31;
-    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < slices; s += (gridDim.x * blockDim.x) >> 5) {
-        const int2 mine = slice_rows[size_t(s) * 32 + lane];
-        const bool long_row = mine.x >= kLongRow;
-        const int row = long_row ? mine.x - kLongRow : mine.x;
-        const long long first = row >= 0 ? rowstr[row] : 0, start = slice_start[s] + 2 * lane;
-        for (int k = 0; k < ((mine.y + 1) & ~1); k++) {
-            const long long from = first + (long_row ? 64LL * (k >> 1) + 2 * lane + (k & 1) : (long long)k);
-            const long long to = start + 64LL * (k >> 1) + (k & 1);
-            const bool in = k < mine.y;
-            const double v = in ? vals[from] : 0.0;
-            a[to] = v;
-            a32[to] = float(v);
-            col[to] = in ? static_cast<unsigned short>(colidx[from]) : 0;
-        }
-    }
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
+         i += (long long)gridDim.x * blockDim.x)
+        out[i] = float(in[i]);
 }
 
 }  // namespace batch
@@ -1135,15 +1035,13 @@ struct cgb_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<SysDesc> desc;
+    std::vector<double> mean_len;
     std::vector<long long> nnz;   // stored entries per system
     std::vector<int> order;       // systems, largest first
     std::vector<int> slots;       // work list of the last launch (system * kMaxTeam + member)
     SysDesc *d_sys = nullptr;
     int *d_slots = nullptr;
-    int *d_rowstr = nullptr;
-    int2 *d_slice_rows = nullptr;
-    long long *d_slice_start = nullptr;
-    unsigned short *d_col = nullptr;
+    int *d_rowstr = nullptr, *d_colidx = nullptr;
     double *d_a = nullptr;
     float *d_a32 = nullptr;
     double *d_x = nullptr, *d_z = nullptr, *d_r = nullptr, *d_q = nullptr, *d_pg = nullptr;
@@ -1169,19 +1067,13 @@ struct cgb_batch {
     double *d_y = nullptr;
     float *d_rg = nullptr, *d_tg = nullptr;
     int *d_fallbacks = nullptr;
-    // 1024 threads: 128 systems of 1400 to 20000 rows, FP64, 104 ms; 512
-    // threads 154 (of 4000 to 12000 rows alone, 24 of them, 35.5 to 37.5 either
-    // way)
-    int block = 1024;
-    int unroll = 4;  // 512-thread shape: 4 or 8 (six pairs) of entries a lane in flight
+    int block = 512;
+    int unroll = 4;  // 512-thread shape: 4 or 8 entries a lane in flight (1024 threads: 4)
     // lane policy: lanes = 32 if mean >= t2, 16 if >= t1, 8 if >= t0, else 4
     double t0 = 16.0, t1 = 40.0, t2 = 96.0;
     // team policy: a system gets 2, 4 or 8 CTAs while its work per CTA is
-    // above team_frac x (the batch's work / the grid's CTAs); 0 = no teams.
-    // Until it is set (cgb_batch_set_team_frac, cgb_batch_tune), the fraction
-    // with the earliest end by team_schedule_us
+    // above team_frac x (the batch's work / the grid's CTAs); 0 = no teams
     double team_frac = 0.5;
-    bool team_frac_set = false;
     int resident = 0;  // CTAs of the last launch's grid (team sizes depend on it)
 };
 
@@ -1204,8 +1096,7 @@ void batch_release(cgb_batch *b)
 {
     if (!b) return;
     cudaSetDevice(b->device);
-    bfree(b->d_sys); bfree(b->d_slots); bfree(b->d_rowstr); bfree(b->d_slice_rows);
-    bfree(b->d_slice_start); bfree(b->d_col); bfree(b->d_a);
+    bfree(b->d_sys); bfree(b->d_slots); bfree(b->d_rowstr); bfree(b->d_colidx); bfree(b->d_a);
     bfree(b->d_a32); bfree(b->d_x); bfree(b->d_z); bfree(b->d_r); bfree(b->d_q); bfree(b->d_pg);
     bfree(b->d_queue); bfree(b->d_team_sync); bfree(b->d_team_part); bfree(b->d_dev_status);
     bfree(b->d_zeta); bfree(b->d_rnorm); bfree(b->d_iters); bfree(b->d_status);
@@ -1218,101 +1109,12 @@ void batch_release(cgb_batch *b)
     delete b;
 }
 
-// The slices of one system (see BatchArgs), appended to `rows` (32 a slice)
-// and `start` (relative to the system's first entry); returns its entries with
-// padding: at most the stored ones plus 32 of the longest row's, since a slice
-// is no wider than any row of the slice before.
-//
-// A row past kLongFactor means (and kLongMin entries) would keep one lane busy
-// while the others wait, so it gets a warp.
-constexpr double kLongFactor = 8.0;
-constexpr int kLongMin = 256;
-
-long long plan_slices(int n, const int *rowstr, std::vector<int2> *rows, std::vector<long long> *start)
-{
-    struct Item {
-        int pairs;  // of the widest lane
-        int first;  // into `sorted`, or the long row
-        bool is_long;
-    };
-    const int bound = int(std::min(1e9, std::max(double(kLongMin), kLongFactor * rowstr[n] / n)));
-    // the other rows by length, longest first (counting sort: stable)
-    int longest = 0;
-    for (int j = 0; j < n; j++) {
-        const int len = rowstr[j + 1] - rowstr[j];
-        if (len <= bound) longest = std::max(longest, len);
-    }
-    std::vector<int> at(size_t(longest) + 2, 0), sorted;
-    std::vector<Item> items;
-    for (int j = 0; j < n; j++) {
-        const int len = rowstr[j + 1] - rowstr[j];
-        if (len <= bound) at[size_t(longest - len) + 1]++;
-        else items.push_back({int((len + 63LL) / 64), j, true});
-    }
-    for (int k = 0; k <= longest; k++) at[k + 1] += at[k];
-    sorted.resize(at[size_t(longest) + 1]);
-    for (int j = 0; j < n; j++) {
-        const int len = rowstr[j + 1] - rowstr[j];
-        if (len <= bound) sorted[at[longest - len]++] = j;
-    }
-    for (int f = 0; f < int(sorted.size()); f += 32)
-        items.push_back({(rowstr[sorted[f] + 1] - rowstr[sorted[f]] + 1) / 2, f, false});
-    std::stable_sort(items.begin(), items.end(), [](const Item &x, const Item &y) { return x.pairs > y.pairs; });
-    long long entries = 0;
-    for (const Item &t : items) {
-        start->push_back(entries);
-        for (int l = 0; l < 32; l++) {
-            int2 mine = make_int2(-1, 0);
-            if (t.is_long) {
-                const int len = rowstr[t.first + 1] - rowstr[t.first];
-                // whole rounds of 64, then what is left from this lane's pair on
-                mine = make_int2(t.first + kLongRow, len / 64 * 2 + std::max(0, std::min(2, len % 64 - 2 * l)));
-            } else if (t.first + l < int(sorted.size())) {
-                const int j = sorted[t.first + l];
-                mine = make_int2(j, rowstr[j + 1] - rowstr[j]);
-            }
-            rows->push_back(mine);
-        }
-        entries += 64LL * t.pairs;
-    }
-    return entries;
-}
-
 int lanes_by_policy(const cgb_batch *b, double mean)
 {
     if (mean >= b->t2) return 32;
     if (mean >= b->t1) return 16;
     if (mean >= b->t0) return 8;
     return 4;
-}
-
-// When the last CTA of `grid` is done if every system ran one product with
-// team_of(i) CTAs, taking systems as the work list hands them out.  A product's
-// time (1024 threads, FP64, measured on systems alone): 2 us + 155 us a million
-// entries on one CTA (25 us at 0.15 million, 491 at 3.1); a team adds 20 us of
-// barriers and of the search vector's exchange to its share (8 CTAs: 30 and
-// 108 us).
-template <typename TeamOf>
-double team_schedule_us(const cgb_batch *b, int grid, TeamOf team_of)
-{
-    std::vector<double> free_at(size_t(grid), 0.0);  // a heap, earliest first
-    const auto later = std::greater<double>();
-    double end = 0.0;
-    for (int i : b->order) {
-        const int t = team_of(i);
-        double start = 0.0;
-        for (int m = 0; m < t; m++) {
-            std::pop_heap(free_at.begin(), free_at.end() - m, later);
-            start = std::max(start, *(free_at.end() - 1 - m));
-        }
-        const double done = start + (t > 1 ? 22.0 : 2.0) + 155e-6 * double(b->nnz[i]) / t;
-        end = std::max(end, done);
-        for (int m = t; m > 0; m--) {
-            *(free_at.end() - m) = done;
-            std::push_heap(free_at.begin(), free_at.end() - m + 1, later);
-        }
-    }
-    return end;
 }
 
 // Lanes per row and team size of every system for a grid of `grid` CTAs,
@@ -1329,27 +1131,14 @@ int apply_policy(cgb_batch *b, int grid)
         total += work[i];
     }
     const double per_cta = total / std::max(grid, 1);
-    auto team_of = [&](int i, double frac) {
-        int t = 1;
-        if (frac > 0.0)
-            while (t < kMaxTeam && 2 * t <= grid && work[i] / t > frac * per_cta) t *= 2;
-        return t;
-    };
-    if (!b->team_frac_set) {
-        double best = 1e300;
-        for (double frac : {0.0, 0.25, 0.35, 0.5, 0.7, 1.0, 1.4, 2.0}) {
-            const double us = team_schedule_us(b, grid, [&](int i) { return team_of(i, frac); });
-            if (us < best) {
-                best = us;
-                b->team_frac = frac;
-            }
-        }
-    }
     b->slots.clear();
     for (int i : b->order) {
         SysDesc &d = b->desc[i];
+        d.lanes = lanes_by_policy(b, b->mean_len[i]);
         d.flanes = b->fmean.empty() ? 4 : lanes_by_policy(b, b->fmean[i]);
-        const int t = team_of(i, b->team_frac);
+        int t = 1;
+        if (b->team_frac > 0.0)
+            while (t < kMaxTeam && 2 * t <= grid && work[i] / t > b->team_frac * per_cta) t *= 2;
         d.team = t;
         for (int m = 0; m < t; m++) b->slots.push_back(i * kMaxTeam + m);
     }
@@ -1368,8 +1157,8 @@ using BatchKernel = void (*)(BatchArgs, const int *, int);
 template <int kMode, bool kTeams>
 BatchKernel pick_kernel(const cgb_batch *b)
 {
-    return b->block > 512 ? batch_kernel<kMode, 1024, 3, kTeams>
-                          : (b->unroll > 4 ? batch_kernel<kMode, 512, 6, kTeams>
+    return b->block > 512 ? batch_kernel<kMode, 1024, 4, kTeams>
+                          : (b->unroll > 4 ? batch_kernel<kMode, 512, 8, kTeams>
                                            : batch_kernel<kMode, 512, 4, kTeams>);
 }
 
@@ -1475,9 +1264,7 @@ int launch(cgb_batch *b, const cgb_batch_params &P, double *ms)
     A.nsys = b->nsys;
     A.sys = b->d_sys;
     A.rowstr = b->d_rowstr;
-    A.slice_rows = b->d_slice_rows;
-    A.slice_start = b->d_slice_start;
-    A.col = b->d_col;
+    A.colidx = b->d_colidx;
     A.a = b->d_a;
     A.a32 = b->d_a32;
     A.x = b->d_x;
@@ -1601,25 +1388,24 @@ int cgb_batch_create(int device, int nsys, const int *n, const int *const *rowst
     b->h_ftcol.resize(nsys);
     b->h_fval.resize(nsys);
     b->h_ftval.resize(nsys);
+    b->mean_len.resize(nsys);
     b->nnz.resize(nsys);
-    long long ro = 0, vo = 0, entries = 0;
-    std::vector<int2> slice_rows;
-    std::vector<long long> slice_start;
+    long long ro = 0, no = 0, vo = 0;
     for (int s = 0; s < nsys; s++) {
         SysDesc &d = b->desc[s];
         d.n = n[s];
         d.row_off = ro;
-        d.slice_off = (long long)slice_start.size();
-        d.entry_off = entries;
-        entries += plan_slices(n[s], rowstr[s], &slice_rows, &slice_start);
-        d.slices = int((long long)slice_start.size() - d.slice_off);
+        d.nnz_off = no;
         d.vec_off = vo;
         d.shift = shift[s];
+        d.lanes = 32;
         d.flanes = 4;
         d.team = 1;
         d.f_row_off = d.f_off = 0;
         b->nnz[s] = rowstr[s][n[s]];
+        b->mean_len[s] = double(rowstr[s][n[s]]) / n[s];
         ro += n[s] + 1;
+        no += rowstr[s][n[s]];
         vo += n[s] + 8;
     }
     std::vector<int> &order = b->order;
@@ -1631,9 +1417,8 @@ int cgb_batch_create(int device, int nsys, const int *n, const int *const *rowst
     bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreate(&b->ev0) == cudaSuccess && cudaEventCreate(&b->ev1) == cudaSuccess &&
               !balloc(&b->d_sys, nsys) && !balloc(&b->d_slots, size_t(nsys) * kMaxTeam) &&
-              !balloc(&b->d_rowstr, rows_total) && !balloc(&b->d_slice_rows, slice_rows.size()) &&
-              !balloc(&b->d_slice_start, slice_start.size()) && !balloc(&b->d_col, entries) &&
-              !balloc(&b->d_a, entries) && !balloc(&b->d_a32, entries) &&
+              !balloc(&b->d_rowstr, rows_total) && !balloc(&b->d_colidx, nnz_total + 64) &&
+              !balloc(&b->d_a, nnz_total + 64) && !balloc(&b->d_a32, nnz_total + 64) &&
               !balloc(&b->d_x, vec_total) && !balloc(&b->d_z, vec_total) &&
               !balloc(&b->d_r, vec_total) && !balloc(&b->d_q, vec_total) &&
               !balloc(&b->d_pg, vec_total) && !balloc(&b->d_queue, 1) &&
@@ -1647,38 +1432,22 @@ int cgb_batch_create(int device, int nsys, const int *n, const int *const *rowst
         batch_release(b);
         return set_error(CGB_ERR_NOMEM, "batch device allocation failed");
     }
-    // a CSR crosses as it is and becomes slices on the device, one system after
-    // another through one staging copy (stream order)
-    long long most = 0;
-    for (int s = 0; s < nsys; s++) most = std::max(most, b->nnz[s]);
-    int *d_cols = nullptr;
-    double *d_vals = nullptr;
-    if (balloc(&d_cols, most) != cudaSuccess || balloc(&d_vals, most) != cudaSuccess) {
-        bfree(d_cols);
-        batch_release(b);
-        return set_error(CGB_ERR_NOMEM, "batch device allocation failed");
-    }
-    ok = cudaMemcpyAsync(b->d_slice_rows, slice_rows.data(), sizeof(int2) * slice_rows.size(), cudaMemcpyHostToDevice,
-                         b->stream) == cudaSuccess &&
-         cudaMemcpyAsync(b->d_slice_start, slice_start.data(), sizeof(long long) * slice_start.size(),
-                         cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
-    for (int s = 0; s < nsys && ok; s++) {
+    for (int s = 0; s < nsys; s++) {
         const SysDesc &d = b->desc[s];
-        const size_t nz = size_t(b->nnz[s]);
-        ok = cudaMemcpyAsync(b->d_rowstr + d.row_off, rowstr[s], sizeof(int) * (n[s] + 1), cudaMemcpyHostToDevice,
-                             b->stream) == cudaSuccess &&
-             cudaMemcpyAsync(d_cols, colidx[s], sizeof(int) * nz, cudaMemcpyHostToDevice, b->stream) == cudaSuccess &&
-             cudaMemcpyAsync(d_vals, a[s], sizeof(double) * nz, cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
-        if (ok)
-            fill_slices<<<4 * b->sms, 256, 0, b->stream>>>(
-                b->d_rowstr + d.row_off, d_cols, d_vals, d.slices, b->d_slice_rows + d.slice_off * 32,
-                b->d_slice_start + d.slice_off, b->d_a + d.entry_off, b->d_a32 + d.entry_off, b->d_col + d.entry_off);
+        const long long nz = rowstr[s][n[s]];
+        // on the batch's stream, so the FP32 conversion below runs after them
+        if (cudaMemcpyAsync(b->d_rowstr + d.row_off, rowstr[s], sizeof(int) * (n[s] + 1),
+                            cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+            cudaMemcpyAsync(b->d_colidx + d.nnz_off, colidx[s], sizeof(int) * nz,
+                            cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+            cudaMemcpyAsync(b->d_a + d.nnz_off, a[s], sizeof(double) * nz, cudaMemcpyHostToDevice,
+                            b->stream) != cudaSuccess) {
+            batch_release(b);
+            return set_error(CGB_ERR_CUDA, "batch upload failed");
+        }
     }
-    ok = ok && cudaGetLastError() == cudaSuccess;
-    const cudaError_t done = cudaStreamSynchronize(b->stream);
-    bfree(d_cols);
-    bfree(d_vals);
-    if (!ok || done != cudaSuccess) {
+    to_fp32_batch<<<4 * b->sms, 256, 0, b->stream>>>(b->d_a, b->d_a32, nnz_total);
+    if (cudaStreamSynchronize(b->stream) != cudaSuccess) {
         batch_release(b);
         return set_error(CGB_ERR_CUDA, "batch set-up failed");
     }
@@ -1717,11 +1486,10 @@ int cgb_batch_solve(cgb_batch *b, const cgb_batch_params *params, double *zeta, 
 }
 
 // Autotuner: times the batch (mode and sizes of `params`) for each block
-// shape {512 threads with 4 or 6 step pairs a lane in flight, 1024 threads}
-// under the team policy that apply_policy finds and, in the learned mode, each
-// lane policy (row-length thresholds for 4/8/16/32 lanes per row of the factor
-// products), then for the best of those the other team policies (no teams,
-// team_frac 0.25 to 1.4), keeps the fastest and reports it.
+// shape {512 threads with 4 or 8 entries a lane in flight, 1024 threads
+// with 4} and each lane policy (row-length thresholds for 4/8/16/32
+// lanes per row), then for the best of those each team policy (no teams,
+// team_frac 0.25, 0.5, 1), keeps the fastest and reports it.
 int cgb_batch_tune(cgb_batch *b, const cgb_batch_params *params, int *block_out, double *t0_out,
                    double *t1_out, double *t2_out, double *best_ms)
 {
@@ -1732,11 +1500,11 @@ int cgb_batch_tune(cgb_batch *b, const cgb_batch_params *params, int *block_out,
         double t0, t1, t2;
         double team_frac;
     };
-    const Cand shapes[] = {{512, 4, 16, 40, 96, -1.0},  {512, 4, 8, 24, 64, -1.0},
-                           {512, 4, 24, 64, 160, -1.0}, {512, 8, 16, 40, 96, -1.0},
-                           {512, 8, 8, 24, 64, -1.0},   {512, 8, 24, 64, 160, -1.0},
-                           {1024, 4, 16, 40, 96, -1.0}, {1024, 4, 8, 24, 64, -1.0},
-                           {512, 4, 1e9, 1e9, 0, -1.0}};
+    const Cand shapes[] = {{512, 4, 16, 40, 96, 0.5},  {512, 4, 8, 24, 64, 0.5},
+                           {512, 4, 24, 64, 160, 0.5}, {512, 8, 16, 40, 96, 0.5},
+                           {512, 8, 8, 24, 64, 0.5},   {512, 8, 24, 64, 160, 0.5},
+                           {1024, 4, 16, 40, 96, 0.5}, {1024, 4, 8, 24, 64, 0.5},
+                           {512, 4, 1e9, 1e9, 0, 0.5}};
     double best = 1e30;
     Cand bc = shapes[0];
     auto trial = [&](const Cand &c) -> int {
@@ -1745,27 +1513,22 @@ int cgb_batch_tune(cgb_batch *b, const cgb_batch_params *params, int *block_out,
         b->t0 = c.t0;
         b->t1 = c.t1;
         b->t2 = c.t2;
-        b->team_frac_set = c.team_frac >= 0.0;  // else the one apply_policy finds
-        if (b->team_frac_set) b->team_frac = c.team_frac;
+        b->team_frac = c.team_frac;
         double ms = 0.0;
         const int st = launch(b, *params, &ms);
         if (st) return st;
         if (ms < best) {
             best = ms;
             bc = c;
-            bc.team_frac = b->team_frac;
         }
         return CGB_OK;
     };
     for (const Cand &c : shapes) {
-        // (the lane policies are the factor products')
-        if (params->mode != CGB_MODE_MIXED_LEARNED && c.t0 != shapes[0].t0) continue;
         const int st = trial(c);
         if (st) return st;
     }
     const Cand shape = bc;
-    for (double f : {0.0, 0.25, 0.5, 0.7, 1.0, 1.4}) {
-        if (f == shape.team_frac) continue;
+    for (double f : {0.0, 0.25, 1.0}) {
         Cand c = shape;
         c.team_frac = f;
         const int st = trial(c);
@@ -1777,7 +1540,6 @@ int cgb_batch_tune(cgb_batch *b, const cgb_batch_params *params, int *block_out,
     b->t1 = bc.t1;
     b->t2 = bc.t2;
     b->team_frac = bc.team_frac;
-    b->team_frac_set = true;
     if (block_out) *block_out = bc.block;
     if (t0_out) *t0_out = bc.t0;
     if (t1_out) *t1_out = bc.t1;
@@ -1910,7 +1672,6 @@ int cgb_batch_set_team_frac(cgb_batch *b, double team_frac)
     if (!b || !(team_frac >= 0.0) || team_frac > 1e6)
         return set_error(CGB_ERR_INVALID, "batch: team_frac must be in [0, 1e6]");
     b->team_frac = team_frac;
-    b->team_frac_set = true;
     return CGB_OK;
 }
 

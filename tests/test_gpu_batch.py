@@ -292,37 +292,3 @@ def test_batch_factor_rows_sorted_and_merged(cgb):
             outs.append(b.solve(niter=5, mode=cgb.MODE_MIXED_LEARNED, tol=1e-12, cgitmax=100))
     assert np.array_equal(outs[0]["zeta"], outs[1]["zeta"])
     assert np.array_equal(outs[0]["iters"], outs[1]["iters"])
-
-
-def test_batch_slices_of_any_rows(cgb, oracle):
-    """The sliced matrices against the oracle's own products where slices can
-    go wrong: fewer rows than a slice, a ragged last slice, no entries beside the
-    diagonal, one row far longer than the others (its own slice, lengths on
-    both sides of a round of 64), unsorted columns; alone and on teams of 8."""
-    rng = np.random.default_rng(5)
-
-    def system(n, extra, long_rows=()):
-        """A varied diagonal plus `extra` random entries a row (a row of long_rows: that many)."""
-        rs, ci, av = [0], [], []
-        for j in range(n):
-            k = dict(long_rows).get(j, extra)
-            cols = rng.choice(n, size=min(k, n), replace=False)
-            cols = cols[cols != j]
-            ci += [j, *cols]
-            av += [-4.0 - 0.05 * (j % 37), *(0.8 / max(1, len(cols)) * rng.uniform(-1, 1, len(cols)))]
-            rs.append(len(ci))
-        return np.array(rs, np.int32), np.array(ci, np.int32), np.array(av)
-
-    systems = [system(31, 0), system(33, 3), system(64, 5), system(700, 4, [(5, 255), (9, 256)]),
-               system(900, 2, [(0, 320), (450, 257), (899, 383), (1, 385), (2, 448)])]
-    shifts = [1.0 + 0.1 * k for k in range(len(systems))]
-    zo = [oracle.conj_grad(rs, ci, a, np.ones(len(rs) - 1))[0][: len(rs) - 1] for rs, ci, a in systems]
-    want = np.array([sh + 1.0 / np.sum(z) for sh, z in zip(shifts, zo)])
-    with cgb.Batch(systems, shifts) as b:
-        outs = []
-        for frac in (0.0, 1e-6):
-            b.set_team_frac(frac)
-            outs.append(b.solve(niter=1))
-            outs.append(b.solve(niter=1, mode=cgb.MODE_MIXED, tol=1e-12, cgitmax=100))
-    for k, out in enumerate(outs):  # FP64: rounding noise; mixed: the parity bar
-        assert np.max(np.abs(out["zeta"] - want) / np.abs(want)) <= (1e-10 if k % 2 else 1e-12)
