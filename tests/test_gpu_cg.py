@@ -403,7 +403,7 @@ def test_column_parts_agree_with_rows(cgb, n):
     assert all(np.array_equal(p, q) for p, q in zip(outs[1][:3], outs[2][:3]))
 
 
-@pytest.mark.parametrize("n", [1023, 1024, 1400, 9001, 24575])
+@pytest.mark.parametrize("n", [1400, 4095, 4096, 9001, 24575])
 def test_small_systems_every_mode(cgb, oracle, n):
     """Below the sliced plan's order the autotuner also has the column parts (6
     of them): whatever it picks, zeta and z agree with the oracle's, and a
