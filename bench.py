@@ -157,6 +157,14 @@ def load_traffic():
     return out, f"ncu capture of this build ({here}), profiles/traffic_per_launch.txt"
 
 
+def sliced_kernel(n, plan):
+    """The FP64 outer-step kernel of a sliced plan at order n: column parts
+    (prefetch or not, one kernel) up to 135680 rows, whole rows beyond."""
+    if n <= 135680:
+        return "outer_step_fp64_parts"
+    return "outer_step_fp64_sliced_pf" if plan["l2_prefetch"] else "outer_step_fp64_sliced"
+
+
 def peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -323,8 +331,8 @@ def class_c_roofline(npbcg, s, n, nnz, niter, shift):
     plan = s.plan()
     peak, peak_kind = peaks()
     if plan["kind"] == "sliced":
-        kernel = "outer_step_fp64_sliced_pf" if plan["l2_prefetch"] else "outer_step_fp64_sliced"
-        spmv_kernel = "spmv_dot_sliced_pf" if plan["l2_prefetch"] else "spmv_dot_sliced"
+        kernel = sliced_kernel(n, plan)
+        spmv_kernel = kernel.replace("outer_step_fp64", "spmv_dot")
     else:
         kernel = f"outer_step_fp64<{plan['lanes_per_row']}>"
         spmv_kernel = f"spmv_dot_row<{plan['lanes_per_row']}>"
@@ -798,7 +806,7 @@ def our_arm(args, rank, world, local_rank):
     # library's stream, algorithmic bytes per launch from outer_step_bytes
     plan = sess.plan()
     if plan["kind"] == "sliced":
-        kernel = "outer_step_fp64_sliced_pf" if plan["l2_prefetch"] else "outer_step_fp64_sliced"
+        kernel = sliced_kernel(n, plan)
     else:
         kernel = f"outer_step_fp64<{plan['lanes_per_row']}>"
     kernel_ms, gap_ms = sess.time_outer_steps(niter, shift)
@@ -845,7 +853,10 @@ def our_arm(args, rank, world, local_rank):
         if not args.no_solver_modes:
             line["solver_modes"] = solver_modes_section(npbcg, device)
             line["roofline_classC"] = line["solver_modes"].pop("roofline_classC")
-        if world == 1 and not args.no_cpu_baseline:
+        ref_lib = os.path.join(ROOT, "oracle", "_ref", f"libref_{CLASS}.so")
+        if world == 1 and not args.no_cpu_baseline and not os.path.exists(ref_lib):
+            line["cpu_baseline"] = {"unavailable": "the reference's sources were not there to build oracle/_ref"}
+        elif world == 1 and not args.no_cpu_baseline:
             nref, nnz_ref, times, rgpu = cpu_reference_run(CPU_SAMPLE_STEPS, gpu_steps=niter)
             sample_bytes = CPU_SAMPLE_STEPS * (CGITMAX + 1) * spmv_bytes(nref, nnz_ref)
             # informative: the reference's own CUDA code on this GPU, the same
