@@ -3,8 +3,7 @@
 // CUDA/MG/mg.cu: main's timed loop :498-508, mg3P :1078-1133).
 //
 // Grids are cubes of side m = 2^k + 2 (one ghost layer a face), x fastest,
-// one buffer per level for u and r (two for the finest u), v on the finest
-// level only.  The operators:
+// one buffer per level for u and r, v on the finest level only.  The operators:
 //   resid   r = v - A u       (:1572-1625)  27-point, a[1] = 0
 //   psinv   u = u + C r       (:1395-1440)  27-point, c[3] = 0
 //   rprj3   s = P^T r         (:1724-1790)  full weighting onto the coarse grid
@@ -904,9 +903,9 @@ struct cgb_mg {
     int m[kMaxLevels + 1] = {};
     double *u[kMaxLevels + 1] = {}, *r[kMaxLevels + 1] = {};
     double *v = nullptr;
-    // the finest level's other u: k_up reads one and writes the other, so the
-    // result of `graph_nit` cycles is u_now
-    double *u_other = nullptr, *u_now = nullptr;
+    // where the run of `graph_nit` cycles leaves the finest u and r: k_up reads
+    // one of u[lt], r[lt] and writes the other (enqueue_region)
+    double *u_now = nullptr, *r_now = nullptr;
     double *d_part = nullptr, *d_norm = nullptr;
     unsigned *d_ticket = nullptr;
     int plus[30] = {}, minus[30] = {};
@@ -950,7 +949,7 @@ void mg_release(cgb_mg *g)
         if (g->u[k]) cudaFree(g->u[k]);
         if (g->r[k]) cudaFree(g->r[k]);
     }
-    for (void *p : {(void *)g->v, (void *)g->u_other, (void *)g->d_part, (void *)g->d_norm, (void *)g->d_ticket})
+    for (void *p : {(void *)g->v, (void *)g->d_part, (void *)g->d_norm, (void *)g->d_ticket})
         if (p) cudaFree(p);
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
@@ -1014,14 +1013,14 @@ dim3 march_grid(const cgb_mg *g, int m, int warps, int extra, int *zc)
     return dim3(unsigned(gx), unsigned(gy), unsigned((n + best_zc - 1) / best_zc));
 }
 
-// r[lt] (when `store`) and r[lt - 1] from the finest u and v
-void launch_down(cgb_mg *g, const double *u, bool store)
+// r (when `store`) and r[lt - 1] from the finest u and v
+void launch_down(cgb_mg *g, const double *u, double *r, bool store)
 {
     const int lt = g->lt, m = g->m[lt];
     int zc = 0;
     const dim3 grid = march_grid(g, m, kWarpsDown, 2, &zc);
     launch(g, store ? k_down<kWarpsDown, true> : k_down<kWarpsDown, false>, grid, dim3(32 * kWarpsDown), u, g->v,
-           g->r[lt], m, g->r[lt - 1], g->m[lt - 1], zc, g->cf);
+           r, m, g->r[lt - 1], g->m[lt - 1], zc, g->cf);
 }
 
 void launch_up(cgb_mg *g, int k, const double *u, const double *v, double *out)
@@ -1048,29 +1047,34 @@ void launch_coarse(cgb_mg *g, int levels, int top, int cycles)
     launch(g, k_coarse, dim3(kClusterCtas), dim3(kClusterThreads), A);
 }
 
-void launch_norm(cgb_mg *g)
+void launch_norm(cgb_mg *g, const double *r)
 {
     const int n = g->m[g->lt] - 2;
     launch(g, k_norm, dim3(unsigned(std::min(kNormBlocks, (n * n + kRowsAhead - 1) / kRowsAhead))), dim3(kNormThreads),
-           g->r[g->lt], g->m[g->lt], g->d_part, g->d_ticket, g->d_norm);
+           r, g->m[g->lt], g->d_part, g->d_ticket, g->d_norm);
 }
 
 // The timed region of main (:498-508): resid, norm, nit x (V-cycle (mg3P,
-// :1078-1133), resid), norm.
-void enqueue_region(cgb_mg *g, int nit)
+// :1078-1133), resid), norm.  The finest u and r are in *uf and *rf after it:
+// above the coarse levels a cycle's k_up reads u and writes the new one over
+// r, which nothing reads between the first norm and the last (k_down walks u
+// and v, and stores r in the last cycle only), so the two buffers change
+// places every cycle.
+void enqueue_region(cgb_mg *g, int nit, double **uf, double **rf)
 {
     const int lt = g->lt, m = g->m[lt];
-    g->u_now = g->u[lt];
+    double *u = g->u[lt], *r = g->r[lt];
     if (lt <= kCoarseLevel) {
-        k_stencil_rb<false><<<stencil_rb_grid(m), dim3(32, kWarpsRB), 0, g->stream>>>(g->u[lt], g->v, g->r[lt], m,
-                                                                                      g->cf);
-        launch_norm(g);
+        k_stencil_rb<false><<<stencil_rb_grid(m), dim3(32, kWarpsRB), 0, g->stream>>>(u, g->v, r, m, g->cf);
+        launch_norm(g, r);
         if (nit > 0) launch_coarse(g, lt, 1, nit);
-        launch_norm(g);
+        launch_norm(g, r);
+        *uf = u;
+        *rf = r;
         return;
     }
-    launch_down(g, g->u_now, true);
-    launch_norm(g);
+    launch_down(g, u, r, true);
+    launch_norm(g, r);
     for (int it = 0; it < nit; it++) {
         for (int k = lt - 1; k > kCoarseLevel; k--) {
             const int mj = g->m[k - 1];
@@ -1078,12 +1082,13 @@ void enqueue_region(cgb_mg *g, int nit)
         }
         launch_coarse(g, kCoarseLevel, 0, 1);
         for (int k = kCoarseLevel + 1; k < lt; k++) launch_up(g, k, nullptr, g->r[k], g->u[k]);
-        double *next = g->u_now == g->u[lt] ? g->u_other : g->u[lt];
-        launch_up(g, lt, g->u_now, g->v, next);
-        g->u_now = next;
-        launch_down(g, g->u_now, it + 1 == nit);
+        launch_up(g, lt, u, g->v, r);
+        std::swap(u, r);
+        launch_down(g, u, r, it + 1 == nit);
     }
-    launch_norm(g);
+    launch_norm(g, r);
+    *uf = u;
+    *rf = r;
 }
 
 // zran3 on the device: the candidates, then the host's choice of the ten
@@ -1223,10 +1228,8 @@ int cgb_mg_create(int device, int lt, int smoother, cgb_mg **out)
     }
     ok = ok && cudaMalloc(&g->v, sizeof(double) * cells(g->m[lt])) == cudaSuccess &&
          cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
-    if (lt > kCoarseLevel)
-        ok = ok && cudaMalloc(&g->u_other, sizeof(double) * cells(g->m[lt])) == cudaSuccess &&
-             cudaMemset(g->u_other, 0, sizeof(double) * cells(g->m[lt])) == cudaSuccess;
     g->u_now = g->u[lt];
+    g->r_now = g->r[lt];
     if (!ok) {
         mg_release(g);
         return set_error(CGB_ERR_NOMEM, "mg: device allocation failed (2^%d grid)", lt);
@@ -1256,8 +1259,9 @@ int cgb_mg_run(cgb_mg *g, int nit, double *rnm2, double *rnmu, double *device_ms
         g->exec = nullptr;
         g->graph_nit = -1;
         cudaGraph_t graph = nullptr;
+        double *u = nullptr, *r = nullptr;
         MG_TRY(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_region(g, nit);
+        enqueue_region(g, nit, &u, &r);
         const cudaError_t e1 = cudaGetLastError();
         const cudaError_t e2 = cudaStreamEndCapture(g->stream, &graph);
         if (e1 != cudaSuccess || e2 != cudaSuccess) {
@@ -1272,6 +1276,8 @@ int cgb_mg_run(cgb_mg *g, int nit, double *rnm2, double *rnmu, double *device_ms
             return set_error(CGB_ERR_CUDA, "mg: graph instantiation: %s", cudaGetErrorString(e3));
         }
         g->graph_nit = nit;
+        g->u_now = u;
+        g->r_now = r;
     }
     // u = 0 on the finest level (main's zero3 before the timed region)
     MG_TRY(cudaMemsetAsync(g->u[lt], 0, sizeof(double) * cells(m), g->stream));
@@ -1297,7 +1303,7 @@ int cgb_mg_read(cgb_mg *g, int which, double *out, long long count)
     const size_t need = cells(g->m[g->lt]);
     if (count < (long long)need) return set_error(CGB_ERR_CAPACITY, "mg: %zu doubles needed", need);
     MG_TRY(cudaSetDevice(g->device));
-    const double *src = which == 0 ? g->u_now : which == 1 ? g->v : g->r[g->lt];
+    const double *src = which == 0 ? g->u_now : which == 1 ? g->v : g->r_now;
     MG_TRY(cudaMemcpy(out, src, sizeof(double) * need, cudaMemcpyDeviceToHost));
     return CGB_OK;
 }

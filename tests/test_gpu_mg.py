@@ -115,6 +115,28 @@ def test_runs_repeat_and_recapture(cgb, oracle):
     assert abs(b["rnm2"] - want["rnm2"]) <= 1e-13 * want["rnm2"]
 
 
+def test_grids_held_and_their_places(cgb, oracle):
+    """A benchmark object holds three finest grids (u, v, r) and the coarse
+    levels' u and r, 0.29 of one together: k_up writes the new u over r.  The
+    two change places every cycle, and the graph captured for another number
+    of cycles leaves them where that number does."""
+    import torch
+    torch.zeros(1, device="cuda")
+    lt = 8
+    with cgb.Mg(5, 0):  # the library's own first allocations
+        before = torch.cuda.mem_get_info()[0]
+        with cgb.Mg(lt, 0):
+            held = (before - torch.cuda.mem_get_info()[0]) / (8.0 * ((1 << lt) + 2) ** 3)
+    assert 3.2 < held < 3.6, held
+    with cgb.Mg(6, 0) as g:
+        for nit in (1, 2, 0, 3):
+            got = g.run(nit)
+            want = oracle.mg_run(6, nit, 0, grids=True)
+            assert np.array_equal(g.grid("u"), want["u"]), nit
+            assert np.array_equal(g.grid("r"), want["r"]), nit
+            assert got["rnmu"] == want["rnmu"], nit
+
+
 def test_invalid_arguments(cgb):
     for lt, sm in ((1, 0), (11, 0), (5, 2)):
         with pytest.raises(cgb.CgbError) as e:
