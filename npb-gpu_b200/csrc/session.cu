@@ -890,7 +890,9 @@ bool make_plan(cgb_session *s, int kind, int lpr, Plan *pl, int prefetch = 0, in
     } else if (kind == kKindSliced) {
         // 32-bit slice offsets: keep the padded copy well below 2^32 entries
         if (!s->sorted || s->d_seg == nullptr || s->nnz > (1LL << 30)) return false;
-        if (s->n < (s->uneven ? 2 * kSliceWidth : kMinPartRows)) return false;
+        // whole rows: two column blocks at least
+        const bool by_parts = s->shape.parts > 0 && !s->uneven;
+        if (s->n < (by_parts ? kMinPartRows : 2 * kSliceWidth)) return false;
         const int grid = std::min(s->prop.multiProcessorCount, s->n);
         if (s->sliced_grid != grid && build_sliced(s, grid) != CGB_OK) return false;
         // more rows a CTA than the accumulators hold: the row-panel
@@ -1180,7 +1182,8 @@ int upload_matrix(cgb_session *s, const int *rowstr, const int *colidx, const do
     s->sorted = false;
     s->uneven = false;
     s->nblk = 0;
-    if (s->n >= (s->opts.spmv_kernel == 0 ? kMinPartRows : 2 * kSliceWidth)) {
+    const bool small_parts = s->opts.spmv_kernel == 0 && s->opts.panel_rows <= 0;
+    if (s->n >= (small_parts ? kMinPartRows : 2 * kSliceWidth)) {
         int st = build_segments_table(s);
         if (st) return st;
     }

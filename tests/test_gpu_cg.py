@@ -445,6 +445,23 @@ def test_uneven_columns_take_whole_rows(cgb):
     assert np.max(np.abs(doubled - ref) / np.abs(ref)) <= 1e-12
 
 
+@pytest.mark.parametrize("n,rows", [(4096, 32), (9001, 4096), (20000, 160), (20000, 4096), (24575, 4096)])
+def test_row_panels_keep_small_systems_on_rows(cgb, n, rows):
+    """Row panels belong to whole rows, which the sliced plan has from 24576
+    rows on; below, an automatic plan with the option is the row plan, whatever
+    its timing (two blocks of whole rows were up to a tenth faster there)."""
+    shift = 10.0 + n / 1500.0
+    rs, ci, a = cgb.makea(n, 15 if n == 20000 else 7, 0.1, shift)
+    with cgb.Session(rs, ci, a, panel_rows=rows) as s:
+        assert s.plan()["kind"] == "row"
+        got = s.power_iterate(2, shift)["zeta"]
+        s.upload(rs, ci, a)
+        assert s.plan()["kind"] == "row"
+    with cgb.Session(rs, ci, a, spmv_kernel=1) as s:
+        want = s.power_iterate(2, shift)["zeta"]
+    assert np.max(np.abs(got - want) / np.abs(want)) <= 1e-12
+
+
 def test_class_d_sliced_row_panels(cgb):
     """Class D (n = 1.5 M, 694 M entries; 10 K rows a CTA) on the sliced
     plan walks row panels; its first outer steps agree with the row plan's
