@@ -594,8 +594,6 @@ int build_segments_table(cgb_session *s)
     const size_t count = size_t(s->nblk + 1) * s->seg_stride;
     if (dev_reserve(&s->d_seg, &s->cap_seg, count) != cudaSuccess)
         return set_error(CGB_ERR_NOMEM, "segment table allocation failed");
-    if (s->shape.parts > 0 && !s->d_parts && dev_alloc(&s->d_parts, kMaxParts * s->vstride) != cudaSuccess)
-        return set_error(CGB_ERR_NOMEM, "product parts allocation failed");
     CUDA_TRY(cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream));
     build_segments<<<4 * s->prop.multiProcessorCount, 256, 0, s->stream>>>(
         s->d_rowstr, s->d_colidx, n, s->nblk, s->shape.width, s->d_seg, s->seg_stride, s->d_flag);
@@ -630,16 +628,13 @@ int chunk_table(int grid, int panels, int nblk, RowsOf rows_of, std::vector<int>
     return total;
 }
 
-// Steps 1-3 of a sliced copy of one matrix over `grid` CTAs: row order per
-// slice, slice offsets, then values (FP64 and/or FP32) and local columns.
-// `seg` is the matrix's segment table; rows are the ranges of row_split (a
-// CTA's, or a group's) or, with `interleave`, every grid-th row.  t->chunk_slice must be set.
-template <typename ST>
-int fill_set(cgb_session *s, int grid, bool interleave, const int *row_split, const int *seg, const int *d_colidx,
-             const ST *vals, int total, bool want64, bool want32, bool want16, SliceSet *t)
+// Steps 1 and 2 of a sliced copy of one matrix over `grid` CTAs: row order per
+// slice, slice offsets, and the copy's entry count.  `seg` is the matrix's
+// segment table; rows are the ranges of row_split (a CTA's, or a group's) or,
+// with `interleave`, every grid-th row.  t->chunk_slice must be set.
+int sort_set(cgb_session *s, int grid, bool interleave, const int *row_split, const int *seg, int total, SliceSet *t)
 {
     const int nblk = t->blocks ? t->blocks : s->nblk;
-    const int bcols = t->block_cols ? t->block_cols : s->shape.width;
     const int nchunks = grid * t->panels * nblk;
     const int ig = interleave ? grid : 0;
     t->interleaved = interleave ? 1 : 0;
@@ -658,6 +653,20 @@ int fill_set(cgb_session *s, int grid, bool interleave, const int *row_split, co
                              s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     t->entries = entries;
+    return CGB_OK;
+}
+
+// Step 3, after sort_set with the same arguments: values (FP64, FP32 and/or
+// BF16) and local columns.
+template <typename ST>
+int fill_set(cgb_session *s, int grid, bool interleave, const int *row_split, const int *seg, const int *d_colidx,
+             const ST *vals, int total, bool want64, bool want32, bool want16, SliceSet *t)
+{
+    const int nblk = t->blocks ? t->blocks : s->nblk;
+    const int bcols = t->block_cols ? t->block_cols : s->shape.width;
+    const int nchunks = grid * t->panels * nblk;
+    const int ig = interleave ? grid : 0;
+    const unsigned entries = unsigned(t->entries);
     if ((want64 && dev_reserve(&t->sval, &t->cap_sval, size_t(entries) + kPad)) ||
         dev_reserve(&t->scol, &t->cap_scol, size_t(entries) + kPad) ||
         (want32 && dev_reserve(&t->sval32, &t->cap_sval32, size_t(entries) + kPad)) ||
@@ -780,21 +789,19 @@ int build_sliced(cgb_session *s, int grid)
     CUDA_TRY(cudaMemcpyAsync(s->d_chunk_slice, chunk_slice.data(), sizeof(int) * chunk_slice.size(),
                              cudaMemcpyHostToDevice, s->stream));
     s->sa.chunk_slice = nullptr;  // the session's table
-    const int st = [&] {
-        SliceSet &t = s->sa;
-        t.chunk_slice = s->d_chunk_slice;
-        const int r = fill_set<double>(s, groups, false, s->d_group_split, s->d_seg, s->d_colidx, s->d_a, total, true,
-                                       s->opts.keep_fp32_copy != 0, false, &t);
-        t.chunk_slice = nullptr;
+    auto with_table = [&](auto step) {
+        s->sa.chunk_slice = s->d_chunk_slice;
+        const int r = step();
+        s->sa.chunk_slice = nullptr;
         return r;
-    }();
+    };
+    int st = with_table([&] { return sort_set(s, groups, false, s->d_group_split, s->d_seg, total, &s->sa); });
     if (st) return st;
-    s->sliced_grid = grid;
-    s->layout_gen++;
     if (h.parts > 0) {
         // a product takes as long as its longest CTA: where the columns are so
         // uneven (a band, an arrow) that one CTA holds a quarter more entries
-        // than the mean, whole rows are the better split
+        // than the mean, whole rows are the better split (known before a
+        // value is copied: the parts' layout is not filled for nothing)
         std::vector<unsigned> off(size_t(total) + 1);
         CUDA_TRY(cudaMemcpyAsync(off.data(), s->sa.off, sizeof(unsigned) * off.size(), cudaMemcpyDeviceToHost,
                                  s->stream));
@@ -808,7 +815,16 @@ int build_sliced(cgb_session *s, int grid)
         plan_part_work(off.data(), chunk_slice.data(), ctas, kSlicedPcgBlock / 32, kBurstPairs, &work);
         CUDA_TRY(cudaMemcpyAsync(s->d_part_work, work.data(), sizeof(unsigned) * work.size(), cudaMemcpyHostToDevice,
                                  s->stream));
+        if (!s->d_parts && dev_alloc(&s->d_parts, kMaxParts * s->vstride) != cudaSuccess)
+            return set_error(CGB_ERR_NOMEM, "product parts allocation failed");
     }
+    st = with_table([&] {
+        return fill_set<double>(s, groups, false, s->d_group_split, s->d_seg, s->d_colidx, s->d_a, total, true,
+                                s->opts.keep_fp32_copy != 0, false, &s->sa);
+    });
+    if (st) return st;
+    s->sliced_grid = grid;
+    s->layout_gen++;
     return CGB_OK;
 }
 
@@ -857,8 +873,9 @@ int ensure_prec_slices(cgb_session *s)
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) st = set_error(CGB_ERR_CUDA, "factor slices: %s", cudaGetErrorString(e));
         else if (unsorted) st = set_error(CGB_ERR_STATE, "factor rows not in ascending column order");
-        else st = fill_set<float>(s, grid, true, s->d_group_split, seg, cols[m], vals[m], total, false, false, true,
-                                  sets[m]);
+        else st = sort_set(s, grid, true, s->d_group_split, seg, total, sets[m]);
+        if (!st) st = fill_set<float>(s, grid, true, s->d_group_split, seg, cols[m], vals[m], total, false, false, true,
+                                      sets[m]);
     }
     dev_free(seg);
     if (st) {

@@ -445,6 +445,24 @@ def test_uneven_columns_take_whole_rows(cgb):
     assert np.max(np.abs(doubled - ref) / np.abs(ref)) <= 1e-12
 
 
+@pytest.mark.parametrize("n,half", [(110000, 40), (130000, 20)])
+def test_uneven_columns_hold_one_layout(cgb, n, half):
+    """A band keeps the memory of a session that was told to take whole rows:
+    of the column parts' layout, which is dropped before it is filled, at most
+    its slices' metadata (1.3 MB; the driver hands out 2 MB at a time)."""
+    import torch
+    torch.zeros(1, device="cuda")
+    m = banded(n, half, 40.0)
+    held = []
+    with cgb.Session(*cgb.makea(1400, 7, 0.1, 10.0)):  # the library's own first allocations
+        for options in ({}, {"panel_rows": 4096}):  # more rows than a CTA has: one panel
+            before = torch.cuda.mem_get_info()[0]
+            with cgb.Session(*m, **options) as s:
+                held.append(before - torch.cuda.mem_get_info()[0])
+                assert s.plan()["kind"] == "row" or s.plan()["panels"] == 1
+    assert abs(held[0] - held[1]) <= 4 << 20, held
+
+
 @pytest.mark.parametrize("n,rows", [(4096, 32), (9001, 4096), (20000, 160), (20000, 4096), (24575, 4096)])
 def test_row_panels_keep_small_systems_on_rows(cgb, n, rows):
     """Row panels belong to whole rows, which the sliced plan has from 24576
