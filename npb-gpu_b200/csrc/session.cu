@@ -1149,6 +1149,12 @@ int choose_plan(cgb_session *s)
     }
     s->plan_main = s->plan_learned = cands[bi];
     if (small && row < cands.size()) s->plan_learned = cands[row];
+    if (small && s->plan_main.kind == kKindRow) {  // nothing walks the sliced candidate again
+        free_sliced(s);
+        dev_free(s->d_parts);
+        dev_free(s->d_seg);
+        s->cap_seg = 0;
+    }
     return apply_plan(s, cands[bi]);
 }
 
@@ -1200,7 +1206,10 @@ int upload_matrix(cgb_session *s, const int *rowstr, const int *colidx, const do
     s->uneven = false;
     s->nblk = 0;
     const bool small_parts = s->opts.spmv_kernel == 0 && s->opts.panel_rows <= 0;
-    if (s->n >= (small_parts ? kMinPartRows : 2 * kSliceWidth)) {
+    const bool small = s->n < 2 * kSliceWidth;
+    // (a small system that keeps the row plan has no use for the table)
+    if (s->n >= (small_parts ? kMinPartRows : 2 * kSliceWidth) &&
+        !(small && same_rows && kept_kind == kKindRow)) {
         int st = build_segments_table(s);
         if (st) return st;
     }

@@ -463,6 +463,26 @@ def test_uneven_columns_hold_one_layout(cgb, n, half):
     assert abs(held[0] - held[1]) <= 4 << 20, held
 
 
+@pytest.mark.parametrize("n", [16000, 24000])
+def test_small_row_plan_keeps_no_sliced_candidate(cgb, n):
+    """Where the autotuner stays on rows (sparse rows of a small system), the
+    session holds what a row session holds, also after an upload of the same
+    rows (within two of the 2 MB pieces that the driver hands out)."""
+    import torch
+    torch.zeros(1, device="cuda")
+    m = cgb.makea(n, 3, 0.1, 20.0)
+    held = []
+    with cgb.Session(*cgb.makea(1400, 7, 0.1, 10.0)):  # the library's own first allocations
+        for options in ({}, {"spmv_kernel": 1}):
+            before = torch.cuda.mem_get_info()[0]
+            with cgb.Session(*m, **options) as s:
+                assert s.plan()["kind"] == "row"
+                held.append(before - torch.cuda.mem_get_info()[0])
+                s.upload(*m)
+                held.append(before - torch.cuda.mem_get_info()[0])
+    assert abs(held[0] - held[2]) <= 4 << 20 and abs(held[1] - held[3]) <= 4 << 20, held
+
+
 @pytest.mark.parametrize("n,rows", [(4096, 32), (9001, 4096), (20000, 160), (20000, 4096), (24575, 4096)])
 def test_row_panels_keep_small_systems_on_rows(cgb, n, rows):
     """Row panels belong to whole rows, which the sliced plan has from 24576
