@@ -50,10 +50,18 @@ constexpr int kKindRow = 1;
 constexpr int kKindSliced = 2;
 constexpr int kKindSlicedPrefetch = 3;  // option and report only: sliced plan with prefetch = 1
 
+// A failed allocation is the caller's to report or to do without: it must not
+// stay behind as the error that the next cudaGetLastError() after a launch
+// returns.
 template <typename T>
 cudaError_t dev_alloc(T **p, size_t count)
 {
-    return cudaMalloc(reinterpret_cast<void **>(p), sizeof(T) * std::max<size_t>(count, 1));
+    const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), sizeof(T) * std::max<size_t>(count, 1));
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        (void)cudaGetLastError();
+    }
+    return e;
 }
 
 // Grow-only buffer: keeps *p when it already holds `count` elements, so a
@@ -65,7 +73,7 @@ cudaError_t dev_reserve(T **p, size_t *cap, size_t count)
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
-    const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), sizeof(T) * std::max<size_t>(count, 1));
+    const cudaError_t e = dev_alloc(p, count);
     if (e == cudaSuccess) *cap = count;
     return e;
 }
@@ -911,7 +919,11 @@ bool make_plan(cgb_session *s, int kind, int lpr, Plan *pl, int prefetch = 0, in
         const bool by_parts = s->shape.parts > 0 && !s->uneven;
         if (s->n < (by_parts ? kMinPartRows : 2 * kSliceWidth)) return false;
         const int grid = std::min(s->prop.multiProcessorCount, s->n);
-        if (s->sliced_grid != grid && build_sliced(s, grid) != CGB_OK) return false;
+        if (s->sliced_grid != grid) {
+            const int st = build_sliced(s, grid);
+            if (st == CGB_ERR_NOMEM) free_sliced(s);  // what fitted of it is of no use
+            if (st) return false;
+        }
         // more rows a CTA than the accumulators hold: the row-panel
         // instances (which have no L2-prefetch form)
         const bool pa = s->sa.panels > 1, pp = pa || s->prec_panels > 1;
@@ -1210,8 +1222,8 @@ int upload_matrix(cgb_session *s, const int *rowstr, const int *colidx, const do
     // (a small system that keeps the row plan has no use for the table)
     if (s->n >= (small_parts ? kMinPartRows : 2 * kSliceWidth) &&
         !(small && same_rows && kept_kind == kKindRow)) {
-        int st = build_segments_table(s);
-        if (st) return st;
+        const int st = build_segments_table(s);
+        if (st && !(small && st == CGB_ERR_NOMEM)) return st;  // a small system has the row plan
     }
     if (same_rows && (kept_kind == kKindRow || (s->sorted && build_sliced(s, kept_grid) == CGB_OK &&
                                                 s->shape == kept_shape))) {

@@ -483,6 +483,32 @@ def test_small_row_plan_keeps_no_sliced_candidate(cgb, n):
     assert abs(held[0] - held[2]) <= 4 << 20 and abs(held[1] - held[3]) <= 4 << 20, held
 
 
+@pytest.mark.parametrize("n,nonzer", [(5000, 40), (30000, 15)])
+def test_row_plan_where_the_sliced_copy_does_not_fit(cgb, n, nonzer):
+    """With room for the matrix but not for a sliced copy beside it, a session
+    runs on the row plan from its first solve on, with the row plan's result."""
+    import torch
+    torch.zeros(1, device="cuda")
+    shift = 2000.0  # above the spectrum of the outer products
+    m = cgb.makea(n, nonzer, 0.1, shift)
+    with cgb.Session(*m) as s:  # every kernel is loaded
+        assert s.plan()["kind"] == "sliced"
+        s.power_iterate(2, shift)
+    before = torch.cuda.mem_get_info()[0]
+    with cgb.Session(*m, spmv_kernel=1) as s:
+        need = before - torch.cuda.mem_get_info()[0]
+        want = s.power_iterate(2, shift)["zeta"]
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - need - (24 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with cgb.Session(*m) as s:
+            assert s.plan()["kind"] == "row"
+            got = s.power_iterate(2, shift)["zeta"]
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert np.max(np.abs(got - want) / np.abs(want)) <= 1e-12
+
+
 @pytest.mark.parametrize("n,rows", [(4096, 32), (9001, 4096), (20000, 160), (20000, 4096), (24575, 4096)])
 def test_row_panels_keep_small_systems_on_rows(cgb, n, rows):
     """Row panels belong to whole rows, which the sliced plan has from 24576
