@@ -641,6 +641,12 @@ struct SlicedSpmvT {
 // the one that began it adds them, in order, after the CTA's barrier.  With whole slices dealt to the warps the longest had 15.8
 // bursts where the mean was 11.5 (n = 75000, 4 parts: 69.8 ms a solve, now 62.3).
 //
+// An FP32 sum is widened after every burst (12 or 20 entries): held over a
+// part, it met up to 27136 columns' entries where whole rows widen after a block
+// of 12288, and dropped twice as much of small entries beside a large one (of 182
+// of 2^-26 beside 1, n = 75000: 8.9e-7, whole rows 4.5e-7, now 1.6e-7; the mixed
+// solve 9.68 -> 9.77 ms at tol 1e-10).
+//
 // (Loading the pairs after while the present ones are used, in two register
 // sets, is slower: 86 to 94 ms a solve at n = 75000 against 66.)  Base: the walk
 // for the preconditioner's factor copies (whole rows).
@@ -718,8 +724,9 @@ struct PartSpmv : Base {
         bool failed = false, staged = false;
         for (; cur.wp >= 0 && !failed; s++) {
             const Slice nxt = slice(s + 1);  // its metadata loads during this slice
-            VT sum = VT(0);
+            double sum = 0.0;
             for (int m = m0; m < cur.wp; m += kU) {
+                VT t = sizeof(VT) == 8 ? VT(sum) : VT(0);
                 P2 av[kU];
                 ushort2 cv[kU];
 #pragma unroll
@@ -746,16 +753,18 @@ struct PartSpmv : Base {
 #pragma unroll
                 for (int u = 0; u < kU; u++) {
                     if (m + u < cur.wp) {
-                        if (CGB_IN_RANGE(cv[u].x, M.width, kCheckGather)) sum = fma_vt(av[u].x, pv[cv[u].x], sum);
-                        if (CGB_IN_RANGE(cv[u].y, M.width, kCheckGather)) sum = fma_vt(av[u].y, pv[cv[u].y], sum);
+                        if (CGB_IN_RANGE(cv[u].x, M.width, kCheckGather)) t = fma_vt(av[u].x, pv[cv[u].x], t);
+                        if (CGB_IN_RANGE(cv[u].y, M.width, kCheckGather)) t = fma_vt(av[u].y, pv[cv[u].y], t);
                     }
                 }
+                if constexpr (sizeof(VT) == 8) sum = t;
+                else sum += double(t);
             }
             const bool valid = cur.row != 0xffffu && CGB_IN_RANGE(row0 + cur.row, M.ncols, kCheckRow);
-            if (valid) dacc = fma(cur.dot, double(sum), dacc);
-            if (m0 > 0) carry[warp * 32 + lane] = double(sum);
-            else if (s == last) carry[(kPartWarps + warp) * 32 + lane] = double(sum);
-            else if (valid) out[cur.row] = double(sum);
+            if (valid) dacc = fma(cur.dot, sum, dacc);
+            if (m0 > 0) carry[warp * 32 + lane] = sum;
+            else if (s == last) carry[(kPartWarps + warp) * 32 + lane] = sum;
+            else if (valid) out[cur.row] = sum;
             m0 = 0;
             cur = nxt;
         }

@@ -403,6 +403,28 @@ def test_column_parts_agree_with_rows(cgb, n):
     assert all(np.array_equal(p, q) for p, q in zip(outs[1][:3], outs[2][:3]))
 
 
+@pytest.mark.parametrize("n,parts", [(75000, 3), (108000, 4)])
+def test_fp32_sums_by_parts_no_coarser_than_whole_rows(cgb, n, parts):
+    """An FP32 row sum by column parts is widened as often as one by whole rows
+    (a block of 12288 columns) at least.  Every row holds one entry of 1 and
+    beside it entries of 2^-26, which an FP32 sum that has met the 1 drops one
+    by one: one CG step from x = 1 gives zeta = 1 / (x.z) = (x.Ax) / n^2, and
+    with it the share dropped, at most that of whole rows."""
+    width = ((n + parts - 1) // parts + 31) & ~31
+    row = (np.arange(parts)[:, None] * width + np.arange(61) * ((n - (parts - 1) * width) // 61)).ravel()
+    vals = np.full(len(row), -2.0**-26)
+    vals[0] = -1.0
+    rs = np.arange(0, n * len(row) + 1, len(row), dtype=np.int32)
+    m = rs, np.tile(row.astype(np.int32), n), np.tile(vals, n)
+    off = []
+    for options in ({}, {"panel_rows": 4096}):  # the second: whole rows, one panel
+        with cgb.Session(*m, spmv_kernel=2, **options) as s:
+            zeta = s.power_iterate(1, 0.0, mode=cgb.MODE_MIXED, tol=1e-30, cgitmax=1, recycle=0)["zeta"][0]
+        off.append(abs(zeta * n / vals.sum() - 1.0))
+    print(f"\nn = {n}: dropped by parts {off[0]:.2e}, by whole rows {off[1]:.2e}")
+    assert off[0] <= off[1] + 2.0**-50
+
+
 @pytest.mark.parametrize("n", [1400, 4095, 4096, 9001, 24575])
 def test_small_systems_every_mode(cgb, oracle, n):
     """Below the sliced plan's order the autotuner also has the column parts (6
