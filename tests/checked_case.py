@@ -52,7 +52,16 @@ def main():
     assert st == 0 and int(d_st.item()) == 0
     out["noalloc_z"] = d_z.cpu().numpy()
     words["noalloc"] = check_word()
-    # sliced plans (class B): both instances, an L2 keep, FP64 and mixed
+    # sliced plans by whole rows (from 135681 rows on): both instances
+    rs, ci, a = npbcg.makea(135681, 5, npbcg.RCOND, 80.0)
+    for kind in (2, 3):
+        with npbcg.Session(rs, ci, a, spmv_kernel=kind) as s:
+            s.set_l2_keep(64e6)
+            out[f"rows{kind}_fp64"] = s.power_iterate(4, 80.0)["zeta"]
+            out[f"rows{kind}_mixed"] = s.power_iterate(4, 80.0, mode=npbcg.MODE_MIXED, tol=1e-12,
+                                                      cgitmax=100)["zeta"]
+        words[f"rows{kind}"] = check_word()
+    # and by column parts (class B): both instances, an L2 keep, FP64 and mixed
     rs, ci, a = npbcg.makea(75000, 13, npbcg.RCOND, 60.0)
     for kind in (2, 3):
         with npbcg.Session(rs, ci, a, spmv_kernel=kind) as s:

@@ -376,14 +376,12 @@ def test_column_parts_agree_with_rows(cgb, n):
     of the columns each) at its smallest order, odd ones, on both sides of one
     part more, its largest and the first by whole rows: every mode's zeta agrees with the row plan's, to 1e-12
     in FP64 (other summation orders) and to the parity bar in the tolerance
-    modes; conj_grad returns the same q = A p, p and z."""
+    modes.  conj_grad's vectors are compared in the next test."""
     rs, ci, a = cgb.makea(n, 5, 0.1, 12.0 + n / 2000.0)
     factor = cgb.jacobi_factor(rs, ci, a)
-    x = 1.0 + 0.5 * np.sin(np.arange(n) * 0.003)
-    outs, vecs = [], []
+    outs = []
     for kind in (1, 2, 3):
         with cgb.Session(rs, ci, a, spmv_kernel=kind) as s:
-            vecs.append(s.conj_grad(x))
             shift = 12.0 + n / 2000.0
             r = [s.power_iterate(4, shift)["zeta"],
                  s.power_iterate(4, shift, mode=cgb.MODE_FP64_TOL, tol=1e-12, cgitmax=100)["zeta"],
@@ -395,12 +393,40 @@ def test_column_parts_agree_with_rows(cgb, n):
     for o in outs[1:]:
         for k, bound in enumerate((1e-12, 1e-10, 1e-10, 1e-10)):
             assert np.max(np.abs(o[k] - outs[0][k]) / np.abs(outs[0][k])) <= bound, (n, k)
-    for v in vecs[1:]:
-        assert np.linalg.norm(v[0] - vecs[0][0]) <= 1e-12 * np.linalg.norm(vecs[0][0])
-        for k in (1, 2):  # p and q: rounding noise by now, of the start's 1e-10 at most
-            assert np.linalg.norm(v[k][:n] - vecs[0][k][:n]) <= 1e-10 * np.linalg.norm(x)
     # the prefetch of the next product's entries changes no bit
     assert all(np.array_equal(p, q) for p, q in zip(outs[1][:3], outs[2][:3]))
+
+
+def unconverged(cgb, n):
+    """A system that 25 CG steps leave far from its solution (diagonals spread
+    over a factor of 300), and a right-hand side: p and q are as large as in the
+    first steps, and no column parts' sum may be missing from them."""
+    shift = 12.0 + n / 2000.0
+    rs, ci, a = cgb.makea(n, 5, 0.1, shift)
+    rows = np.repeat(np.arange(n), np.diff(rs))
+    d = rows == ci
+    a[d] -= 300.0 * shift * rows[d] / n
+    return rs, ci, a, 1.0 + 0.5 * np.sin(np.arange(n) * 0.003)
+
+
+@pytest.mark.parametrize("n", [24576, 30011, 75037, 81408, 81409, 135680, 135681])
+def test_column_parts_return_every_vector(cgb, oracle, n):
+    """conj_grad by column parts returns z, p, q = A p and r = A z as the oracle
+    does.  Seen between the oracle and sums in another order (NumPy, all three
+    sizes tried): z 2e-14, p and q 1.2e-13, r 1.2e-14, each of its own norm; the
+    bounds are a hundred times that.  Entry n, which no product touches, comes
+    back as it went in."""
+    rs, ci, a, x = unconverged(cgb, n)
+    want = oracle.conj_grad(rs, ci, a, x)
+    assert np.linalg.norm(want[2][:n]) > 1e-3 * np.linalg.norm(x)  # q has not converged
+    for kind in (2, 3):
+        with cgb.Session(rs, ci, a, spmv_kernel=kind) as s:
+            for _ in range(2):
+                got = s.conj_grad(x)
+                for k, bound in enumerate((2e-12, 1.2e-11, 1.2e-11, 1.2e-12)):
+                    off = np.linalg.norm(got[k][:n] - want[k][:n])
+                    assert off <= bound * np.linalg.norm(want[k][:n]), (kind, "zpqr"[k])
+                assert [v[n] for v in got[:4]] == [0.0, 1.0, 0.0, 1.0]
 
 
 @pytest.mark.parametrize("n,parts", [(75000, 3), (108000, 4)])
@@ -427,10 +453,10 @@ def test_fp32_sums_by_parts_no_coarser_than_whole_rows(cgb, n, parts):
 
 @pytest.mark.parametrize("n", [1400, 4095, 4096, 9001, 24575])
 def test_small_systems_every_mode(cgb, oracle, n):
-    """Below the sliced plan's order the autotuner also has the column parts (6
-    of them): whatever it picks, zeta and z agree with the oracle's, and a
-    learned solve between two FP64 ones (which may run on another plan) changes
-    neither."""
+    """Below 24576 rows: whatever plan the autotuner picks (the row plan below
+    4096 rows; from there on it also has six column parts), zeta and z agree
+    with the oracle's, and a learned solve between two FP64 ones (which may run
+    on another plan) changes neither."""
     shift = 12.0 + n / 2000.0
     rs, ci, a = cgb.makea(n, 6, 0.1, shift)
     zo, *_ = oracle.conj_grad(rs, ci, a, np.ones(n))
@@ -441,11 +467,46 @@ def test_small_systems_every_mode(cgb, oracle, n):
         s.set_preconditioner(*cgb.jacobi_factor(rs, ci, a))
         learned = s.power_iterate(3, shift, mode=cgb.MODE_MIXED_LEARNED, tol=1e-12, cgitmax=100)["zeta"]
         again = s.power_iterate(3, shift)["zeta"]
-        assert s.plan()["kind"] in ("row", "sliced")
+        assert n >= 4096 or s.plan()["kind"] == "row"
     assert np.linalg.norm(z[:n] - zo[:n]) <= 1e-12 * np.linalg.norm(zo[:n])
     assert np.array_equal(first, again)
     for other in (mixed, learned):
         assert np.max(np.abs(other - first) / np.abs(first)) <= 1e-10
+
+
+@pytest.mark.parametrize("n,nonzer", [(14000, 11), (22001, 13)])
+def test_six_column_parts(cgb, oracle, n, nonzer):
+    """Six column parts, which no option forces: at class A and a larger order
+    they are a fifth to a third faster than the row plan, so the autotuner picks them.
+    Every mode's zeta and an unconverged conj_grad's vectors agree with the
+    row plan's and the oracle's (bounds: test_column_parts_return_every_vector)."""
+    shift = 10.0 + n / 1400.0
+    rs, ci, a = cgb.makea(n, nonzer, 0.1, shift)
+    rows = np.repeat(np.arange(n), np.diff(rs))
+    d = rows == ci
+    b = a.copy()
+    b[d] -= 300.0 * shift * rows[d] / n
+    x = 1.0 + 0.5 * np.sin(np.arange(n) * 0.003)
+    want = oracle.conj_grad(rs, ci, b, x)
+    zetas = []
+    for kind in (1, 0):
+        with cgb.Session(rs, ci, a, spmv_kernel=kind) as s:
+            plan = s.plan()
+            assert plan["kind"] == ("row" if kind else "sliced"), plan
+            r = [s.power_iterate(4, shift)["zeta"],
+                 s.power_iterate(4, shift, mode=cgb.MODE_FP64_TOL, tol=1e-12, cgitmax=100)["zeta"],
+                 s.power_iterate(4, shift, mode=cgb.MODE_MIXED, tol=1e-12, cgitmax=100)["zeta"]]
+            s.set_preconditioner(*cgb.jacobi_factor(rs, ci, a))
+            r.append(s.power_iterate(4, shift, mode=cgb.MODE_MIXED_LEARNED, tol=1e-12, cgitmax=100)["zeta"])
+            zetas.append(r)
+            if kind == 0:
+                s.upload(rs, ci, b)  # the same rows: the plan stays
+                assert s.plan()["kind"] == "sliced"
+                got = s.conj_grad(x)
+    for k, bound in enumerate((1e-12, 1e-10, 1e-10, 1e-10)):
+        assert np.max(np.abs(zetas[1][k] - zetas[0][k]) / np.abs(zetas[0][k])) <= bound, k
+    for k, bound in enumerate((2e-12, 1.2e-11, 1.2e-11, 1.2e-12)):
+        assert np.linalg.norm(got[k][:n] - want[k][:n]) <= bound * np.linalg.norm(want[k][:n]), "zpqr"[k]
 
 
 def test_uneven_columns_take_whole_rows(cgb):

@@ -3,8 +3,8 @@
 single-system SpMVs is tested against its buffer, a failure recorded in a
 check word and the access skipped (no trap).  Run over the row plan, a CSR
 with an odd entry count (its last pair), the allocation-free entry on
-unpadded caller buffers, both sliced instances with an L2 keep, and the
-FP64, mixed and learned modes: no index may leave its buffer, and the
+unpadded caller buffers, both sliced instances with an L2 keep by whole rows
+and by column parts, and the FP64, mixed and learned modes: no index may leave its buffer, and the
 outputs must equal the normal build's bit for bit (the checks change no
 arithmetic)."""
 import os
