@@ -549,6 +549,13 @@ int cgb_ft_destroy(cgb_ft *f);
  * niter in [1, 64]; either output may be NULL. */
 int cgb_ft_run(cgb_ft *f, int niter, double *sums, double *device_ms);
 
+/* Self-test of the fused y and x pass's bounded wait (fields of 100 MB and
+ * more): one x tile waits limit_ns for y tiles that nobody writes, and the
+ * status the host reads back is returned (CGB_ERR_TIMEOUT expected;
+ * CGB_ERR_STATE where the field has no such pass).  The fields are untouched
+ * and the next run starts over. */
+int cgb_ft_selftest_wait(cgb_ft *f, long long limit_ns);
+
 /* After a run: which 0 u0 (the evolved field in Fourier space), 1 u1 (the
  * last inverse transform), 2 the twiddle factors (nx ny nz doubles);
  * count: doubles available at out (2 nx ny nz for u0 and u1). */

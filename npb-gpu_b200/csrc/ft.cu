@@ -538,7 +538,7 @@ constexpr int kTilePoints = 4096;
 constexpr int kTileThreads = kTilePoints / 16;
 constexpr long long kWaitNs = 2000000000LL;
 
-__device__ __forceinline__ bool wait_count(const int *count, int want, const int *failed)
+__device__ __forceinline__ bool wait_count(const int *count, int want, const int *failed, long long limit_ns)
 {
     unsigned long long t0 = 0;
     for (unsigned spins = 0;; spins++) {
@@ -549,14 +549,15 @@ __device__ __forceinline__ bool wait_count(const int *count, int want, const int
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             if (t0 == 0) t0 = t;
-            if ((long long)(t - t0) > kWaitNs || *(volatile const int *)failed) return false;
+            if ((long long)(t - t0) > limit_ns || *(volatile const int *)failed) return false;
         }
     }
 }
 
 template <int NX, int NY, int SIGN>
 __global__ void __launch_bounds__(kTileThreads, 2)
-    k_fft_yx(double2 *u, const double2 *__restrict__ W, int wscale_x, int wscale_y, int nz, int lag, PlaneSync s)
+    k_fft_yx(double2 *u, const double2 *__restrict__ W, int wscale_x, int wscale_y, int nz, int lag, PlaneSync s,
+             long long limit_ns)
 {
     constexpr int LX = kTilePoints / NX, LY = kTilePoints / NY, TP = NX * NY / kTilePoints;
     extern __shared__ double2 sbuf[];
@@ -581,7 +582,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
             plane = g - nz;
             x_axis = 1;
         }
-        if (threadIdx.x == 0 && x_axis && !wait_count(s.done + plane, TP, s.failed)) {
+        if (threadIdx.x == 0 && x_axis && !wait_count(s.done + plane, TP, s.failed, limit_ns)) {
             atomicExch(s.failed, 1);
             stop = 1;
         }
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(kPoints) k_checksum(const double2 *u1, int nx,
 
 using FftKernel = void (*)(const double2 *, double2 *, double2 *, const double *, const double2 *, int, int, int,
                            int, int, int);
-using FusedKernel = void (*)(double2 *, const double2 *, int, int, int, int, PlaneSync);
+using FusedKernel = void (*)(double2 *, const double2 *, int, int, int, int, PlaneSync, long long);
 
 struct Launch {
     FftKernel k = nullptr;
@@ -820,7 +821,7 @@ void enqueue_benchmark(cgb_ft *f, int niter)
         run_pass(f, f->inv[2], 2, f->u0, f->u1, it, it == niter);
         if (f->inv_yx.k) {
             f->inv_yx.k<<<f->inv_yx.grid, kTileThreads, f->inv_yx.smem, f->stream>>>(
-                f->u1, f->W, f->maxdim / f->nx, f->maxdim / f->ny, f->nz, f->inv_yx.lag, sync);
+                f->u1, f->W, f->maxdim / f->nx, f->maxdim / f->ny, f->nz, f->inv_yx.lag, sync, kWaitNs);
         } else {
             run_pass(f, f->inv[1], 1, f->u1, f->u1);
             run_pass(f, f->inv[0], 0, f->u1, f->u1);
@@ -940,6 +941,28 @@ int cgb_ft_run(cgb_ft *f, int niter, double *sums, double *device_ms)
             sums[2 * (it - 1) + 1] = h[it].y;
         }
     if (device_ms) *device_ms = ms;
+    return CGB_OK;
+}
+
+int cgb_ft_selftest_wait(cgb_ft *f, long long limit_ns)
+{
+    if (!f || limit_ns <= 0 || limit_ns > 10000000000LL)
+        return set_error(CGB_ERR_INVALID, "ft: limit_ns must be in (0, 1e10]");
+    if (!f->inv_yx.k) return set_error(CGB_ERR_STATE, "ft: this field takes the y and x axes apart");
+    FT_TRY(cudaSetDevice(f->device));
+    const cudaStream_t st = f->stream;
+    const PlaneSync sync = plane_sync(f);
+    // only the last item is left to hand out, an x tile; no plane has a y tile
+    const int last = 2 * f->nz * (f->nx * f->ny / kTilePoints) - 1;
+    FT_TRY(cudaMemsetAsync(f->sync, 0, sizeof(int) * size_t(f->nz + 2), st));
+    FT_TRY(cudaMemcpyAsync(sync.ticket, &last, sizeof(int), cudaMemcpyHostToDevice, st));
+    f->inv_yx.k<<<f->inv_yx.grid, kTileThreads, f->inv_yx.smem, st>>>(
+        f->u1, f->W, f->maxdim / f->nx, f->maxdim / f->ny, f->nz, f->inv_yx.lag, sync, limit_ns);
+    FT_TRY(cudaGetLastError());
+    int failed = 0;
+    FT_TRY(cudaMemcpyAsync(&failed, sync.failed, sizeof(int), cudaMemcpyDeviceToHost, st));
+    FT_TRY(cudaStreamSynchronize(st));
+    if (failed) return set_error(CGB_ERR_TIMEOUT, "ft: a plane's y tiles were not done within the wait limit");
     return CGB_OK;
 }
 

@@ -222,6 +222,7 @@ _SIGNATURES = {
                                      ctypes.POINTER(ctypes.c_void_p)]),
     "cgb_ft_destroy": (ctypes.c_int, [ctypes.c_void_p]),
     "cgb_ft_run": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, _F64, ctypes.POINTER(ctypes.c_double)]),
+    "cgb_ft_selftest_wait": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_longlong]),
     "cgb_ft_read": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, _F64, ctypes.c_longlong]),
     "cgb_host_alloc": (ctypes.c_int, [ctypes.POINTER(ctypes.c_void_p), ctypes.c_longlong]),
     "cgb_host_free": (ctypes.c_int, [ctypes.c_void_p]),
@@ -1184,6 +1185,10 @@ class Ft:
         t = ctypes.c_double()
         _check(lib().cgb_ft_run(self._h, int(niter), sums, ctypes.byref(t)))
         return dict(sums=[(sums[2 * i], sums[2 * i + 1]) for i in range(niter)], device_ms=t.value)
+
+    def selftest_wait(self, limit_ns):
+        """The status of the fused pass's bounded-wait self-test."""
+        return lib().cgb_ft_selftest_wait(self._h, int(limit_ns))
 
     def read(self, which):
         """'u0' or 'u1' (complex, shape (nz, ny, nx)) or 'twiddle' (float, same shape)."""

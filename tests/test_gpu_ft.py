@@ -41,10 +41,13 @@ def test_ft_shapes_match_oracle(cgb, oracle, dims):
     check_against_oracle(cgb, oracle, *dims)
 
 
-@pytest.mark.parametrize("dims", [(128, 128, 512, 1), (1024, 128, 64, 1), (128, 1024, 64, 1), (512, 256, 64, 2)])
+@pytest.mark.parametrize("dims", [(128, 128, 512, 1), (1024, 128, 64, 1), (128, 1024, 64, 1), (512, 256, 64, 2),
+                                  (256, 128, 256, 1), (256, 256, 128, 1), (256, 1024, 32, 1), (512, 512, 32, 1),
+                                  (1024, 1024, 32, 1), (1024, 512, 32, 1), (1024, 256, 32, 1), (128, 256, 256, 1),
+                                  (128, 512, 128, 1), (256, 512, 64, 1), (512, 128, 128, 1), (512, 1024, 32, 1)])
 def test_ft_fused_planes_match_oracle(cgb, oracle, dims):
     """Fields beyond 100 MB take the y and x axes in one kernel (a plane's x
-    tiles wait for its y tiles): the shortest and longest sides it is compiled
+    tiles wait for its y tiles): every pair of the sides that it is compiled
     for, few and many tiles a plane."""
     assert 16 * dims[0] * dims[1] * dims[2] >= 100 << 20
     check_against_oracle(cgb, oracle, *dims)
@@ -71,6 +74,21 @@ def test_ft_repeatable_and_invalid(cgb):
         with pytest.raises(cgb.CgbError) as e:
             cgb.Ft(*dims)
         assert e.value.status == cgb.ERR_INVALID
+
+
+def test_fused_plane_wait_runs_out(cgb):
+    """A plane's x tile whose y tiles nobody writes gives up after its limit and
+    the host reads the status; the fields are untouched and the object runs on.
+    A field whose axes run apart has no such wait."""
+    with cgb.Ft(128, 128, 512) as f:
+        first = f.run(2)["sums"]
+        u1 = f.read("u1")
+        assert f.selftest_wait(0) == cgb.ERR_INVALID
+        assert f.selftest_wait(1_000_000) == cgb.ERR_TIMEOUT
+        assert np.array_equal(f.read("u1"), u1)
+        assert f.run(2)["sums"] == first
+    with cgb.Ft(64, 64, 64) as f:
+        assert f.selftest_wait(1_000_000) == cgb.ERR_STATE
 
 
 def test_reference_gpu_ft_agrees(cgb):
