@@ -5,9 +5,12 @@ multiply-adds, so each operator's output grid -- interior and ghost layer --
 must equal the oracle's (oracle/mg_oracle.c, pinned to the reference's
 verification norms) bit for bit, and so must the whole benchmark's u and r
 after the V-cycles.  Only the residual norm's sum runs in another order:
-relative 1e-13 against the oracle.  Every class S-C must verify against the
+relative 1e-13 against the oracle, and 1e-14 against the sum of the grid's
+squares rounded once where the oracle's own serial sum is further off.  Every class S-C must verify against the
 reference's norms at the reference's own epsilon, 1e-8 (mg.cu:528-543).
 """
+import math
+
 import numpy as np
 import pytest
 
@@ -88,12 +91,14 @@ def test_fused_cycles_bitwise(cgb, oracle, lt, nit, smoother):
         got = g.run(nit)
         assert np.array_equal(g.grid("u"), want["u"])
         assert np.array_equal(g.grid("r"), want["r"])
-    # the oracle adds m = 8^lt squares one after another: m 2^-53 of the sum at
-    # most, half of it after the root (3.5e-13 seen of 9.3e-10 at lt = 8); the
-    # kernel's tree, at most 64 roundings deep with its rows, comes on top
-    bound = (8**lt / 2 + 64) * 2.0**-53
-    assert abs(got["rnm2"] - want["rnm2"]) <= bound * want["rnm2"]
     assert got["rnmu"] == want["rnmu"]
+    # The kernel adds the rounded squares at most 77 deep (lt = 8: 56 rows a
+    # block, a tree of 256 threads, five blocks a thread, the tree again), each
+    # addition within 2^-53 of a sum of positive terms; the root halves that:
+    # 4.3e-15 with the quotient and the root themselves.
+    r = want["r"].reshape(3 * ((1 << lt) + 2,))[1:-1, 1:-1, 1:-1]
+    exact = math.sqrt(math.fsum((r * r).ravel()) / 8.0**lt)
+    assert abs(got["rnm2"] - exact) <= 1e-14 * exact
 
 
 @pytest.mark.parametrize("cls", ["S", "W", "A", "B", pytest.param("C", marks=pytest.mark.slow)])
