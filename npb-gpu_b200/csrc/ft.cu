@@ -7,9 +7,9 @@
 // A transform along one axis is one kernel: a CTA stages a tile of L lines
 // of that axis in shared memory (rows of L consecutive x values for the y
 // and z axes, so every row is one coalesced run; L whole x lines for the x
-// axis) and transforms every line by radix-8 Stockham stages (a 4 or a 2
-// last), each stage's butterflies in registers: the first stage reads its
-// points from the field, the last writes its outputs to the field, and the
+// axis) and transforms every line by Stockham stages of radix 8 and 16 (4 for
+// the rest of 32 points), each stage's butterflies in registers: the first
+// stage reads its points from the field, the last writes its outputs to the field, and the
 // stages between exchange through shared memory.  So each axis costs one
 // read and one write of the field, and where the y and the x axis share a
 // kernel (k_fft_yx) the two together do.  The inverse transform's first axis
@@ -163,14 +163,6 @@ __device__ __forceinline__ double2 rot90(double2 z)
     return SIGN > 0 ? make_double2(-z.y, z.x) : make_double2(z.y, -z.x);
 }
 
-template <int SIGN>
-__device__ __forceinline__ void dft2(double2 *x)
-{
-    const double2 t = x[0];
-    x[0] = cadd(t, x[1]);
-    x[1] = csub(t, x[1]);
-}
-
 // y_k = sum_j x_j w^(jk), w = exp(2 pi i SIGN / 4), in place, natural order
 template <int SIGN>
 __device__ __forceinline__ void dft4(double2 *x)
@@ -245,10 +237,10 @@ __device__ __forceinline__ void dft16(double2 *x)
 template <int R, int SIGN>
 __device__ __forceinline__ void dft(double2 *x)
 {
+    static_assert(R == 4 || R == 8 || R == 16, "radix_of");
     if constexpr (R == 16) dft16<SIGN>(x);
     else if constexpr (R == 8) dft8<SIGN>(x);
-    else if constexpr (R == 4) dft4<SIGN>(x);
-    else dft2<SIGN>(x);
+    else dft4<SIGN>(x);
 }
 
 // Radix of the stage that has `rest` points a sub-transform left to do: 16
@@ -337,13 +329,11 @@ __device__ __forceinline__ void twiddle_dft(double2 *v, int j, const double2 *__
             v[5] = cmul(v[5], cmul(w1, w4));
             v[6] = cmul(v[6], cmul(w2, w4));
             v[7] = cmul(v[7], cmul(w3, w4));
-        } else if constexpr (R == 4) {
+        } else {
             const double2 w1 = root(1), w2 = root(2);
             v[1] = cmul(v[1], w1);
             v[2] = cmul(v[2], w2);
             v[3] = cmul(v[3], cmul(w1, w2));
-        } else {
-            v[1] = cmul(v[1], root(1));
         }
     }
     dft<R, SIGN>(v);
@@ -521,7 +511,7 @@ __global__ void __launch_bounds__(Tile<N, AXIS, TP>::T, Tile<N, AXIS, TP>::CTAS)
 // The y and then the x axis in one kernel, in place, for fields beyond the
 // L2: a plane's y tiles are written and its x tiles read a few planes later,
 // while the plane is still in L2, so the two axes together read and write
-// HBM once.  Work items (tiles of 4096 points, 512 threads, two CTAs an SM)
+// HBM once.  Work items (tiles of 4096 points, 256 threads, two CTAs an SM)
 // are handed out by a ticket in this order: the y tiles of planes 0 .. lag-1,
 // then those of plane lag + i and the x tiles of plane i in turn, then the
 // last planes' x tiles.  An x tile waits until its plane's y tiles are
@@ -534,8 +524,8 @@ __global__ void __launch_bounds__(Tile<N, AXIS, TP>::T, Tile<N, AXIS, TP>::CTAS)
 // this one 469; at 256 x 256 x 128 (134 MB) 978 and 942; at 512 x 256 x 256
 // and 20 iterations 11.27 and 11.04 ms, at 512^3 52.2 and 49.6.
 constexpr long long kLargeBytes = 100LL << 20;
-constexpr int kTilePoints = 4096;
-constexpr int kTileThreads = kTilePoints / 16;
+constexpr int kTilePoints = kLargeTile;
+constexpr int kTileThreads = kTilePoints / kPerThread;
 constexpr long long kWaitNs = 2000000000LL;
 
 __device__ __forceinline__ bool wait_count(const int *count, int want, const int *failed, long long limit_ns)
