@@ -322,7 +322,9 @@ int cgb_time_outer_steps(cgb_session *s, int niter, double shift, double *kernel
  * block (the FP64 and FP32 SpMVs of the matrix; not the factor products);
  * lanes per row (row kind), grid, block, dynamic shared memory
  * bytes, and the stored entries of the layout the SpMV streams (nnz for the
- * CSR, nnz plus slice padding for the sliced copy).  Any output may be NULL. */
+ * CSR, nnz plus slice padding for the sliced copy).  Any output may be NULL.
+ * (Below 24576 rows the preconditioned mode stays on the fastest row plan,
+ * whatever the others run on.) */
 int cgb_plan_info(cgb_session *s, int *kind, int *lanes_per_row, int *grid, int *block,
                   long long *smem_bytes, long long *layout_entries);
 
@@ -340,6 +342,10 @@ int cgb_set_l2_keep(cgb_session *s, double bytes);
  * more above about 2100 rows a CTA, or below opts->panel_rows); 0 and 0 for
  * the row plan.  No counterpart in the reference. */
 int cgb_plan_panels(cgb_session *s, int *panels, int *prec_panels);
+/* Column parts of the sliced plan: CTAs in groups of `*parts` share their
+ * rows, a part of the columns each; 0 where every CTA computes whole rows, and
+ * for the row plan.  No counterpart in the reference. */
+int cgb_plan_parts(cgb_session *s, int *parts);
 
 /* The checked build (lib/libcgb_checked.so, compiled with -DCGB_CHECKED)
  * tests every index of the single-system SpMVs against its buffer and skips

@@ -1069,8 +1069,8 @@ static __global__ void build_segments(const int *__restrict__ rowstr,
 // (counting sort on min(len, 255)), 32 to a slice; srow gets the local row of
 // each (slice, lane), 0xffff for the tail; slice_width the longest segment,
 // rounded up to even.
-// Placement order within a bin does not matter: each row is summed by one
-// lane in its CSR order wherever it lands.
+// Each row is summed by one lane in its CSR order wherever it lands; rows of a
+// bin keep their order (below).
 // Rows of CTA c: row_split[c] + i for i < row_split[c+1] - row_split[c], or
 // (interleaved, grid G) c + G i for i < interleaved_rows(n, c, G).  Row
 // panel k of `panels` takes the local rows [panel_begin(rows, k), panel_begin(

@@ -1939,6 +1939,13 @@ int cgb_plan_panels(cgb_session *s, int *panels, int *prec_panels)
     return CGB_OK;
 }
 
+int cgb_plan_parts(cgb_session *s, int *parts)
+{
+    if (!s || !parts) return set_error(CGB_ERR_INVALID, "bad arguments");
+    *parts = s->plan_main.kind == kKindSliced ? s->shape.parts : 0;
+    return CGB_OK;
+}
+
 int cgb_set_l2_keep(cgb_session *s, double bytes)
 {
     if (!s || !(bytes >= 0.0) || bytes > 1e12) return set_error(CGB_ERR_INVALID, "bytes must be in [0, 1e12]");

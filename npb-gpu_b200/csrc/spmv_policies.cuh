@@ -1,6 +1,6 @@
-// spmv_policies.cuh -- the two SpMV policies of the persistent CG kernels.
+// spmv_policies.cuh -- the SpMV policies of the persistent CG kernels.
 //
-// Both compute out[j] = (A v)[j] for the rows [row0, row1) the CTA owns and
+// They compute out[j] = (A v)[j] for the rows [row0, row1) the CTA owns and
 // return this thread's share of dotv . out (FP64).  They are generic in the
 // value type VT: double for the FP64 solver (the reference's precision,
 // cg.cu:691-697), float for the FP32 SpMV of the mixed-precision solver
@@ -31,6 +31,8 @@
 //                  end -- deterministic.  The preconditioner's factor copies
 //                  gather a BF16 vector (FP32 row sums), so a staged block
 //                  spans twice the columns.
+//   PartSpmv       the same slices, but CTAs in groups share their rows and each
+//                  stages one part of the vector whole: see there.
 #pragma once
 
 #include <cuda_bf16.h>

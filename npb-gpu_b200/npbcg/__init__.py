@@ -163,6 +163,7 @@ _SIGNATURES = {
                                       ctypes.POINTER(ctypes.c_int)] +
                        [ctypes.POINTER(ctypes.c_double)] * 4),
     "cgb_plan_l2_keep": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]),
+    "cgb_plan_parts": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
     "cgb_plan_panels": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int),
                                        ctypes.POINTER(ctypes.c_int)]),
     "cgb_check_status": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
@@ -425,10 +426,12 @@ class Session:
         _check(lib().cgb_plan_l2_keep(self._h, ctypes.byref(keep)))
         pa, pf = ctypes.c_int(), ctypes.c_int()
         _check(lib().cgb_plan_panels(self._h, ctypes.byref(pa), ctypes.byref(pf)))
+        parts = ctypes.c_int()
+        _check(lib().cgb_plan_parts(self._h, ctypes.byref(parts)))
         return dict(kind={1: "row", 2: "sliced", 3: "sliced"}.get(kind, kind), l2_prefetch=kind == 3,
                     l2_keep_mb=keep.value / 1e6, lanes_per_row=lpr, grid=grid, block=block,
                     smem=smem.value, layout_entries=entries.value, panels=pa.value,
-                    prec_panels=pf.value)
+                    prec_panels=pf.value, parts=parts.value)
 
     def set_l2_keep(self, nbytes):
         """Bytes of the sliced matrix stream kept in L2 across products
@@ -1007,14 +1010,27 @@ def mg_apply(op, m, in1, in2=None, out=None, smoother=0, device=0):
     return res
 
 
+MG_COARSE_LEVEL = 5  # mg.cu's k_coarse: every level up to 32^3 in one launch
+
+
 def mg_region_bytes(lt, nit):
     """Algorithmic bytes of the MG timed region (resid, norm, nit x (V-cycle,
-    resid), norm): every grid an operator reads or writes, counted once per
-    operator, ghost layers included; a level-k grid is (2^k + 2)^3 doubles."""
+    resid), norm): every grid a pass reads or writes, counted once per pass,
+    ghost layers included; a level-k grid is (2^k + 2)^3 doubles.  Above 32^3 a
+    pass is a fused march (mg.cu): interp + resid + psinv, and resid + rprj3,
+    which writes r the first and the last time only; up to 32^3 an operator."""
     c = {k: 8.0 * ((1 << k) + 2) ** 3 for k in range(1, lt + 1)}
-    cycle = sum(c[k] + c[k - 1] for k in range(2, lt + 1))          # rprj3
+    coarse = min(lt, MG_COARSE_LEVEL)
+    cycle = sum(c[k] + c[k - 1] for k in range(2, lt))                # rprj3
     cycle += c[1] + 3 * c[1]                                          # zero, psinv
-    cycle += sum(c[k - 1] + c[k] + 3 * c[k] + 3 * c[k] for k in range(2, lt))  # interp, resid, psinv
+    inner = range(2, coarse + 1 if lt > coarse else lt)
+    cycle += sum(c[k - 1] + c[k] + 3 * c[k] + 3 * c[k] for k in inner)  # interp, resid, psinv
+    if lt > coarse:
+        cycle += sum(c[k - 1] + 2 * c[k] for k in range(coarse + 1, lt))
+        cycle += c[lt - 1] + 3 * c[lt]
+        cycle += 2 * c[lt] + c[lt - 1]
+        return nit * cycle + (3 * c[lt] + c[lt - 1]) + (c[lt] if nit else 0) + 2 * c[lt]
+    cycle += c[lt] + c[lt - 1]                                        # rprj3 from the finest
     cycle += c[lt - 1] + 2 * c[lt] + 3 * c[lt] + 3 * c[lt]            # interp (adding), resid, psinv
     cycle += 3 * c[lt]                                                # the main loop's resid
     return 3 * c[lt] + 2 * c[lt] + nit * cycle

@@ -10,6 +10,7 @@
     python npb-gpu_b200/npbcg/profile_case.py --what ep --ep-class B
     python npb-gpu_b200/npbcg/profile_case.py --what is --is-class B
     python npb-gpu_b200/npbcg/profile_case.py --what ft --ft-class B
+    python npb-gpu_b200/npbcg/profile_case.py --cls A --what train --reps 3
 
 `spmv` launches the standalone FP64 SpMV+dot kernel `reps` times (after one
 warm-up launch); `solve` runs one power iteration of `niter` outer steps;
@@ -19,8 +20,9 @@ from this process; `mg` runs the MG benchmark's timed region (niter
 V-cycles) of an MG class once after one warm-up run; `ep` runs the EP
 kernel of an EP class once; `is` runs the IS benchmark (one untimed and ten
 timed ranking passes, the full check) of an IS class once; `ft` runs the FT
-benchmark's timed region of an FT class once after one warm-up run.  Each
-prints one JSON line.
+benchmark's timed region of an FT class once after one warm-up run; `train`
+takes the network's loss and gradients on a CG class's matrix `reps` times
+after one warm-up.  Each prints one JSON line.
 """
 import argparse
 import json
@@ -35,7 +37,7 @@ def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--cls", default="B", choices=sorted(npbcg.CLASSES))
     ap.add_argument("--what", default="spmv",
-                    choices=["spmv", "solve", "sweep", "batch", "barrier", "part", "mg", "ep", "is", "ft"])
+                    choices=["spmv", "solve", "sweep", "batch", "barrier", "part", "mg", "ep", "is", "ft", "train"])
     ap.add_argument("--ep-class", default="B", choices=sorted(npbcg.EP_CLASSES),
                     help="ep: the EP class")
     ap.add_argument("--ft-class", default="B", choices=sorted(npbcg.FT_CLASSES),
@@ -113,7 +115,20 @@ def main():
     rs, ci, av = npbcg.makea(c["n"], c["nonzer"], npbcg.RCOND, c["shift"])
     n, nnz = c["n"], len(av)
     out = {"cls": a.cls, "n": n, "nnz": nnz, "what": a.what}
-    if a.what == "sweep":
+    if a.what == "train":
+        import time
+
+        import numpy as np
+        model = npbcg.Gnn()
+        model.load()
+        probes = np.random.default_rng(1).standard_normal((n, 32)).astype(np.float32)
+        with model.graph(rs, ci, av) as g:
+            model.loss_grad(g, probes)
+            t0 = time.perf_counter()
+            for _ in range(a.reps):
+                loss, _ = model.loss_grad(g, probes)
+            out.update(loss=float(loss), ms_host=(time.perf_counter() - t0) * 1e3 / a.reps)
+    elif a.what == "sweep":
         rows = []
         configs = [(1, l) for l in (8, 16, 32)] + [(2, 0)]
         for kind, lanes in configs:

@@ -5,7 +5,7 @@ checksums, ft.cu:1655-1810): every iteration's checksum within relative
 1e-13, the last inverse transform u1 and the evolved field u0 within 1e-12
 of their largest element, the twiddle factors within an ulp (CUDA's exp
 against the C library's, the same argument).  Shapes cover every line
-length 32 .. 2048 and the radix-4 and radix-2 last stages.  Every class
+length 32 .. 2048 and the last stages of radix 4, 8 and 16.  Every class
 S-D must verify at the reference's 1e-12.
 """
 import numpy as np
