@@ -95,7 +95,8 @@ typedef struct cgb_options {
                                  a multiple of 32 (0 = as many as its shared accumulators
                                  hold, about 2100).  A CTA with more rows walks them in row
                                  panels, every column block once per panel (class D: 5
-                                 panels); every row is summed in the same order, the fused dot
+                                 panels).  Rows are whole then (no column parts); a row is
+                                 summed in the same order at every panel size, the fused dot
                                  products add rows in another order.  No counterpart
                                  in the reference. */
 } cgb_options;
