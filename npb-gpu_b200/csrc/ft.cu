@@ -389,9 +389,13 @@ __device__ __forceinline__ void mid_stages(double2 *s, const double2 *__restrict
 // Lines a CTA: about TP points a tile, 2 .. 16 lines (x lines); y and z lines
 // at least 8 (a row of L consecutive x values is the run each strided row
 // read fetches: 128 bytes) and at most 32, and at most 8192 points.  TP is
-// 4096 for fields beyond the L2 and 2048 for those within it, which have too
+// 4096 for fields beyond the L2; 2048 for those within it, which have too
 // few tiles to fill the SMs evenly: 128^3 points 247 -> 220 us for 6
-// iterations, 512 x 256 x 256 11.27 (4096) against 11.39 ms.
+// iterations, 512 x 256 x 256 11.27 (4096) against 11.39 ms; and 512 for fields
+// of up to 2^20 points, whose 2048-point tiles leave SMs without one (8
+// iterations, 512 against 2048: 32 x 64 x 32 86.0 and 92.1 us, 128 x 128 x 32 127
+// and 131, 128 x 128 x 64 171 and 184; the same at 2^20 and below in every
+// other shape or better, at 2^21 between 2 % better and 2 % worse).
 constexpr int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 template <int N, int AXIS, int TP>
 struct Tile {
@@ -399,7 +403,8 @@ struct Tile {
     static constexpr int T = N * L / kPerThread;
     static constexpr int CTAS = 8192 / (N * L) < 1 ? 1 : 8192 / (N * L);  // 128 registers a thread
 };
-constexpr int kLargeTile = 4096, kSmallTile = 2048;
+constexpr int kLargeTile = 4096, kSmallTile = 2048, kTinyTile = 512;
+constexpr long long kTinyPoints = 1 << 20;
 
 // One tile of one axis of the transform, AXIS 0 (x), 1 (y), 2 (z): L lines
 // of N points, point n of line l at base + n sn + l sl, by T threads.  in and
@@ -700,15 +705,19 @@ Launch pick_tile(int n)
     case 256: return make_launch<256, AXIS, SIGN, EVOLVE, TP>();
     case 512: return make_launch<512, AXIS, SIGN, EVOLVE, TP>();
     case 1024: return make_launch<1024, AXIS, SIGN, EVOLVE, TP>();
-    case 2048: return make_launch<2048, AXIS, SIGN, EVOLVE, TP>();
+    case 2048:  // with sides of 32 at least, such a field is never a tiny one
+        if constexpr (TP != kTinyTile) return make_launch<2048, AXIS, SIGN, EVOLVE, TP>();
+        return Launch{};
     default: return Launch{};
     }
 }
 
 template <int AXIS, int SIGN, bool EVOLVE>
-Launch pick(int n, bool large)
+Launch pick(int n, long long points)
 {
-    return large ? pick_tile<AXIS, SIGN, EVOLVE, kLargeTile>(n) : pick_tile<AXIS, SIGN, EVOLVE, kSmallTile>(n);
+    if (points <= kTinyPoints) return pick_tile<AXIS, SIGN, EVOLVE, kTinyTile>(n);
+    if (points * (long long)sizeof(double2) < kLargeBytes) return pick_tile<AXIS, SIGN, EVOLVE, kSmallTile>(n);
+    return pick_tile<AXIS, SIGN, EVOLVE, kLargeTile>(n);
 }
 
 }  // namespace ft
@@ -846,13 +855,12 @@ int cgb_ft_create(int device, int nx, int ny, int nz, cgb_ft **out)
     f->maxdim = std::max(nx, std::max(ny, nz));
     f->nt = (long long)nx * ny * nz;
     f->k2max = (nx / 2) * (nx / 2) + (ny / 2) * (ny / 2) + (nz / 2) * (nz / 2);
-    const bool large = is_large(f);
-    f->fwd[0] = pick<0, 1, false>(nx, large);
-    f->fwd[1] = pick<1, 1, false>(ny, large);
-    f->fwd[2] = pick<2, 1, false>(nz, large);
-    f->inv[0] = pick<0, -1, false>(nx, large);
-    f->inv[1] = pick<1, -1, false>(ny, large);
-    f->inv[2] = pick<2, -1, true>(nz, large);
+    f->fwd[0] = pick<0, 1, false>(nx, f->nt);
+    f->fwd[1] = pick<1, 1, false>(ny, f->nt);
+    f->fwd[2] = pick<2, 1, false>(nz, f->nt);
+    f->inv[0] = pick<0, -1, false>(nx, f->nt);
+    f->inv[1] = pick<1, -1, false>(ny, f->nt);
+    f->inv[2] = pick<2, -1, true>(nz, f->nt);
     bool ok = true;
     for (const Launch *a : {&f->fwd[0], &f->fwd[1], &f->fwd[2], &f->inv[0], &f->inv[1], &f->inv[2]})
         ok = ok && a->k &&

@@ -41,6 +41,16 @@ def test_ft_shapes_match_oracle(cgb, oracle, dims):
     check_against_oracle(cgb, oracle, *dims)
 
 
+@pytest.mark.parametrize("dims", [(32, 32, 32, 3), (32, 64, 32, 2), (64, 256, 64, 1), (512, 32, 32, 1), (32, 32, 512, 1),
+                                  (1024, 32, 32, 1), (32, 256, 128, 1),  # tiles of 512 points, to 2^20
+                                  (128, 128, 256, 1), (64, 512, 64, 1), (512, 64, 128, 1), (256, 64, 256, 1),
+                                  (32, 1024, 128, 1), (32, 64, 2048, 1)])  # of 2048
+def test_ft_tile_sizes_match_oracle(cgb, oracle, dims):
+    """Every line length in the tiles of fields up to 2^20 points and of fields
+    up to 100 MB, the smallest and the largest field of either."""
+    check_against_oracle(cgb, oracle, *dims)
+
+
 @pytest.mark.parametrize("dims", [(128, 128, 512, 1), (1024, 128, 64, 1), (128, 1024, 64, 1), (512, 256, 64, 2),
                                   (256, 128, 256, 1), (256, 256, 128, 1), (256, 1024, 32, 1), (512, 512, 32, 1),
                                   (1024, 1024, 32, 1), (1024, 512, 32, 1), (1024, 256, 32, 1), (128, 256, 256, 1),
